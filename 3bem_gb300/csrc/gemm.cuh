@@ -11,8 +11,9 @@
 // so a column is len contiguous values: B columns have length k, D columns
 // length m.
 //
-// CTA: 256 threads, tile BM x 64 (BM = 128 or 64: the choice that pads m the
-// least), each thread an (BM / 16) x 4 block of outputs.  A launch with too
+// FP32 (grouped_gemm_kernel): CTA of 256 threads, tile BM x 64 (BM = 128 or
+// 64: the choice that pads m the least), each thread an (BM / 16) x 4 block of
+// outputs.  FP64: dgemm_warp_kernel below, tiles of one warp.  A launch with too
 // few tiles to fill the GPU splits K over blockIdx.z (partial products added
 // atomically).  K runs in steps of
 // BK through two shared-memory buffers: the next step's global loads are in
@@ -27,9 +28,10 @@ namespace tbem {
 
 constexpr int GM_BN = 64, GM_THREADS = 256;
 
-// GEMM_WAVES: deterministic accumulation -- the groups run in conflict-free
-// waves (no output written twice within a wave), each wave with GEMM_ADD.
-enum GemmMode { GEMM_STORE = 0, GEMM_ADD = 1, GEMM_ATOMIC = 2, GEMM_WAVES = 3 };
+// GEMM_ADD needs groups that write every output at most once (else the sum is
+// a race): sets that add several products into one output run through a
+// SlotPlan (plan.h) or atomically.
+enum GemmMode { GEMM_STORE = 0, GEMM_ADD = 1, GEMM_ATOMIC = 2 };
 
 template <typename T>
 struct GemmArgs {
@@ -58,18 +60,15 @@ __device__ __forceinline__ void atomic_add_t<double>(double* p, double v) { atom
 template <>
 __device__ __forceinline__ void atomic_add_t<float>(float* p, float v) { atomicAdd(p, v); }
 
-// K step: 16 for FP32; 8 for FP64 (keeps the two buffers within 48 KB)
-template <typename T>
-struct GemmK {
-    static constexpr int BK = sizeof(T) == 4 ? 16 : 8;
-};
+constexpr int GM_BK = 16;  // K step
 
 // One output tile (column tile `tile`, row tile `mtile`, K split `kz`) of a
 // grouped GEMM (the body of grouped_gemm_kernel).
-template <typename T, int BM>
-__device__ __forceinline__ void gemm_tile(const GemmArgs<T>& a, int tile, int mtile, int kz)
+template <int BM>
+__device__ __forceinline__ void gemm_tile(const GemmArgs<float>& a, int tile, int mtile, int kz)
 {
-    constexpr int BN = GM_BN, BK = GemmK<T>::BK;
+    using T = float;
+    constexpr int BN = GM_BN, BK = GM_BK;
     constexpr int TM = BM / 16, TN = BN / 16;  // outputs per thread (rows x columns)
     constexpr int PA = BM + 4, PB = BN + 4;     // padded row lengths of the shared tiles
     constexpr int NA = BM * BK / GM_THREADS;    // A elements loaded per thread per step
@@ -160,23 +159,11 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs<T>& a, int tile, int mt
             T av[TM], bv[TN];
 #pragma unroll
             for (int i = 0; i < TM; i += 4) {
-                if constexpr (sizeof(T) == 4) {
-                    const float4 v = *reinterpret_cast<const float4*>(&As[buf][kk][ty * TM + i]);
-                    av[i] = v.x; av[i + 1] = v.y; av[i + 2] = v.z; av[i + 3] = v.w;
-                } else {
-                    const double2 v0 = *reinterpret_cast<const double2*>(&As[buf][kk][ty * TM + i]);
-                    const double2 v1 = *reinterpret_cast<const double2*>(&As[buf][kk][ty * TM + i + 2]);
-                    av[i] = v0.x; av[i + 1] = v0.y; av[i + 2] = v1.x; av[i + 3] = v1.y;
-                }
+                const float4 v = *reinterpret_cast<const float4*>(&As[buf][kk][ty * TM + i]);
+                av[i] = v.x; av[i + 1] = v.y; av[i + 2] = v.z; av[i + 3] = v.w;
             }
-            if constexpr (sizeof(T) == 4) {
-                const float4 v = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * TN]);
-                bv[0] = v.x; bv[1] = v.y; bv[2] = v.z; bv[3] = v.w;
-            } else {
-                const double2 v0 = *reinterpret_cast<const double2*>(&Bs[buf][kk][tx * TN]);
-                const double2 v1 = *reinterpret_cast<const double2*>(&Bs[buf][kk][tx * TN + 2]);
-                bv[0] = v0.x; bv[1] = v0.y; bv[2] = v1.x; bv[3] = v1.y;
-            }
+            const float4 v = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * TN]);
+            bv[0] = v.x; bv[1] = v.y; bv[2] = v.z; bv[3] = v.w;
 #pragma unroll
             for (int i = 0; i < TM; i++)
 #pragma unroll
@@ -211,10 +198,10 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs<T>& a, int tile, int mt
     }
 }
 
-template <typename T, int BM>
-__global__ void __launch_bounds__(GM_THREADS) grouped_gemm_kernel(const GemmArgs<T> a)
+template <int BM>
+__global__ void __launch_bounds__(GM_THREADS) grouped_gemm_kernel(const GemmArgs<float> a)
 {
-    gemm_tile<T, BM>(a, blockIdx.x, blockIdx.y, blockIdx.z);
+    gemm_tile<BM>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // Row tile for m rows: the one that pads m the least (128 on a tie).
@@ -222,6 +209,110 @@ inline int gemm_bm(int m)
 {
     const int p128 = (m + 127) / 128 * 128, p64 = (m + 63) / 64 * 64;
     return p64 < p128 ? 64 : 128;
+}
+
+// ---------------------------------------------------------------- FP64 GEMM
+//
+// GB300 issues two FP64 FMAs per SM and clock (1.25 TFLOP/s), so an FP64
+// translation is paced by that pipe alone: a 64 x 64 tile with K = 297 keeps
+// one SM busy for 0.3 ms, and every padded row or column costs as much as a
+// real one.  So the work is cut as finely as a warp allows: one warp owns 8
+// rows x 4 TN columns (lane: row lane % 8, columns lane / 8 + 4 j), TN = 1 ..
+// 4 being what the tile's columns need, so at most 7 rows and 3 columns per
+// group are padding, and four warps of a CTA take neighbouring row blocks of
+// the same columns (their B values meet in L1).  Operands are loaded straight
+// from global memory (L1 keeps the lines over 16 depths): a warp needs 24
+// values per 64-FMA-clock step at TN = 4, far below what L1 and L2 deliver,
+// so there is no staging and no barrier.  The next U depths are in registers
+// while the current U are multiplied; U = 16 / TN keeps about 1,000 pipe
+// clocks of work in flight over an L2 latency.
+//
+// Every output is one chain over ascending depth (in GEMM_ATOMIC launches of
+// too few warps K is split over blockIdx.z).
+constexpr int DG_WARPS = 4, DG_ROWS = 8;
+
+template <int TN>
+__device__ __forceinline__ void dgemm_warp(const GemmArgs<double>& a, int g, int col0, int ncols, int m0, int kb,
+                                           int kend)
+{
+    constexpr int U = TN == 1 ? 16 : TN == 2 ? 8 : 4;
+    const int lane = threadIdx.x % 32, lr = lane % DG_ROWS, lc = lane / DG_ROWS;
+    const int M = a.m, K = a.k, nrhs = a.nrhs;
+    const long pair0 = a.g_pair0[g];
+    const long ldb = (long)nrhs * K, ldd = (long)nrhs * M;
+    const int row = m0 + lr;
+    // rows and columns past the end read the last valid one and are not stored
+    const int rrow = min(row, M - 1);
+    const long astep = a.trans ? a.lda : 1;
+    const double* __restrict__ ap = a.A[g] + (a.trans ? (long)rrow : (long)rrow * a.lda) + (long)kb * astep;
+    const double* bp[TN];
+#pragma unroll
+    for (int j = 0; j < TN; j++) {
+        const int c = min(col0 + lc + 4 * j, ncols - 1);
+        const int p = c / nrhs, r = c - p * nrhs;
+        bp[j] = a.B + (long)a.in_cell[pair0 + p] * ldb + (long)r * K + kb;
+    }
+    double acc[TN];
+#pragma unroll
+    for (int j = 0; j < TN; j++) acc[j] = 0.0;
+
+    const int n = kend - kb, nfull = n / U;
+    double av[U], bv[TN][U];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            av[u] = ap[(long)(k0 + u) * astep];
+#pragma unroll
+            for (int j = 0; j < TN; j++) bv[j][u] = bp[j][k0 + u];
+        }
+    };
+    if (nfull > 0) load(0);
+    for (int q = 0; q < nfull; q++) {
+        double ac[U], bc[TN][U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            ac[u] = av[u];
+#pragma unroll
+            for (int j = 0; j < TN; j++) bc[j][u] = bv[j][u];
+        }
+        if (q + 1 < nfull) load((q + 1) * U);
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int j = 0; j < TN; j++) acc[j] = fma(ac[u], bc[j][u], acc[j]);
+    }
+    for (int k = nfull * U; k < n; k++) {
+        const double x = ap[(long)k * astep];
+#pragma unroll
+        for (int j = 0; j < TN; j++) acc[j] = fma(x, bp[j][k], acc[j]);
+    }
+    if (row >= M) return;
+#pragma unroll
+    for (int j = 0; j < TN; j++) {
+        const int c = col0 + lc + 4 * j;
+        if (c >= ncols) continue;
+        const int p = c / nrhs, r = c - p * nrhs;
+        double* d = a.D + (long)a.out_cell[pair0 + p] * ldd + (long)r * M + row;
+        if (a.mode == GEMM_STORE) *d = acc[j];
+        else if (a.mode == GEMM_ADD) *d += acc[j];
+        else atomic_add_t<double>(d, acc[j]);
+    }
+}
+
+// bn: columns per tile (4, 8 or 16); blockIdx.x the column tile, .y the group
+// of DG_WARPS row blocks, .z the K split
+__global__ void __launch_bounds__(32 * DG_WARPS) dgemm_warp_kernel(const GemmArgs<double> a, int bn);
+
+// Columns per warp tile for `cols` columns of m rows on `sms` SMs: as wide as
+// possible (fewer operand loads per FMA) while every SM gets 16 warps; below
+// that a launch is one chain of K dependent FMAs per output, and the narrow
+// tile makes the chain the shortest.
+inline int dgemm_bn(long cols, int m, int sms)
+{
+    const long rows = (m + DG_ROWS - 1) / DG_ROWS;
+    for (int bn : {16, 8})
+        if (rows * ((cols + bn - 1) / bn) >= 16L * sms) return bn;
+    return 4;
 }
 
 }  // namespace tbem

@@ -113,71 +113,66 @@ void GemmSet::upload(const void* pool, size_t esz)
     std::vector<const void*> ptrs(A_off.size());
     for (size_t g = 0; g < A_off.size(); g++)
         ptrs[g] = static_cast<const char*>(pool) + A_off[g] * esz;
-    d_A.upload(ptrs);
-    d_pair0.upload(pair0);
-    d_npairs.upload(npairs);
-    d_in.upload(in_cell);
-    d_out.upload(out_cell);
+    table = PackedTable();
+    const size_t oa = table.add(ptrs), op = table.add(pair0), on = table.add(npairs), oi = table.add(in_cell),
+                 oo = table.add(out_cell);
+    table.upload();
+    d_A = table.at<const void*>(oa);
+    d_pair0 = table.at<long>(op);
+    d_npairs = table.at<int>(on);
+    d_in = table.at<int>(oi);
+    d_out = table.at<int>(oo);
     tiles.clear();
 }
 
-// Greedy wave assignment: a group goes one wave after the latest wave that
-// already writes any of its output cells, so no wave writes a cell twice.
-void GemmSet::build_waves()
+__global__ void __launch_bounds__(32 * DG_WARPS) dgemm_warp_kernel(const GemmArgs<double> a, int bn)
 {
-    int max_cell = 0;
-    for (int c : out_cell) max_cell = std::max(max_cell, c);
-    std::vector<int> last(max_cell + 1, -1);
-    wave_of.assign(npairs.size(), 0);
-    n_waves = 0;
-    for (size_t g = 0; g < npairs.size(); g++) {
-        int w = 0;
-        for (long p = pair0[g]; p < pair0[g] + npairs[g]; p++) w = std::max(w, last[out_cell[p]] + 1);
-        for (long p = pair0[g]; p < pair0[g] + npairs[g]; p++) last[out_cell[p]] = w;
-        wave_of[g] = w;
-        n_waves = std::max(n_waves, w + 1);
-    }
+    const int m0 = (blockIdx.y * DG_WARPS + threadIdx.x / 32) * DG_ROWS;
+    if (m0 >= a.m) return;
+    const int g = a.tile_group[blockIdx.x], col0 = a.tile_col0[blockIdx.x];
+    const int ncols = a.g_npairs[g] * a.nrhs;
+    const int kb = blockIdx.z * a.kchunk, kend = min(a.k, kb + a.kchunk);
+    const int tn = (min(bn, ncols - col0) + 3) / 4;
+    if (tn == 1) dgemm_warp<1>(a, g, col0, ncols, m0, kb, kend);
+    else if (tn == 2) dgemm_warp<2>(a, g, col0, ncols, m0, kb, kend);
+    else if (tn == 3) dgemm_warp<3>(a, g, col0, ncols, m0, kb, kend);
+    else dgemm_warp<4>(a, g, col0, ncols, m0, kb, kend);
 }
 
 template <typename T>
 void GemmSet::run_rect(const T* B, T* D, int m, int k, int lda, int nrhs, int trans, int mode,
-                       cudaStream_t s, long* launches, bool tables_only)
+                       cudaStream_t s, long* launches)
 {
     if (empty()) return;
-    const bool waves = mode == GEMM_WAVES;
-    if (waves && wave_of.empty()) build_waves();
-    auto it = tiles.find(nrhs);
+    int dev = 0, sms = 0;
+    TBEM_CK(cudaGetDevice(&dev));
+    TBEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    constexpr bool f64 = sizeof(T) == 8;
+    const int bn = f64 ? dgemm_bn(total_pairs() * nrhs, m, sms) : GM_BN;
+    const std::pair<int, int> key{nrhs, bn};
+    auto it = tiles.find(key);
     if (it == tiles.end()) {
-        // tiles ordered by wave (a single wave when waves are not used)
-        std::vector<int> tg, tc, start;
-        const int nw = wave_of.empty() ? 1 : n_waves;
-        for (int w = 0; w < nw; w++) {
-            start.push_back((int)tg.size());
-            for (size_t g = 0; g < npairs.size(); g++) {
-                if (!wave_of.empty() && wave_of[g] != w) continue;
-                int ncols = npairs[g] * nrhs;
-                for (int c = 0; c < ncols; c += GM_BN) {
-                    tg.push_back((int)g);
-                    tc.push_back(c);
-                }
+        std::vector<int> tg, tc;
+        for (size_t g = 0; g < npairs.size(); g++) {
+            const int ncols = npairs[g] * nrhs;
+            for (int c = 0; c < ncols; c += bn) {
+                tg.push_back((int)g);
+                tc.push_back(c);
             }
         }
-        start.push_back((int)tg.size());
-        auto& e = tiles[nrhs];
+        auto& e = tiles[key];
         e.first.upload(tg);
         e.second.upload(tc);
-        wave_tile_start[nrhs] = start;
-        it = tiles.find(nrhs);
+        it = tiles.find(key);
     }
-    if (tables_only) return;
     GemmArgs<T> a;
-    a.A = reinterpret_cast<const T* const*>(d_A.p);
-    a.g_pair0 = d_pair0.p;
-    a.g_npairs = d_npairs.p;
+    a.A = reinterpret_cast<const T* const*>(d_A);
+    a.g_pair0 = d_pair0;
+    a.g_npairs = d_npairs;
     a.tile_group = it->second.first.p;
     a.tile_col0 = it->second.second.p;
-    a.in_cell = d_in.p;
-    a.out_cell = d_out.p;
+    a.in_cell = d_in;
+    a.out_cell = d_out;
     a.B = B;
     a.D = D;
     a.m = m;
@@ -185,40 +180,31 @@ void GemmSet::run_rect(const T* B, T* D, int m, int k, int lda, int nrhs, int tr
     a.lda = lda;
     a.nrhs = nrhs;
     a.trans = trans;
-    a.mode = waves ? GEMM_ADD : mode;
-    const std::vector<int>& st = wave_tile_start[nrhs];
-    const int nw = (int)st.size() - 1;
-    if (!waves && nw != 1) throw Error(TBEM_ERR_STATE, "a wave-ordered GEMM set run without waves");
-    int dev = 0, sms = 0;
-    TBEM_CK(cudaGetDevice(&dev));
-    TBEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    for (int w = 0; w < nw; w++) {
-        const int nt = st[w + 1] - st[w];
-        if (nt == 0) continue;
-        a.tile_group = it->second.first.p + st[w];
-        a.tile_col0 = it->second.second.p + st[w];
-        const int bm = gemm_bm(m);
-        const long ctas = (long)nt * ((m + bm - 1) / bm);
-        // split K when the tiles fill less than two CTAs per SM and the
-        // accumulation is atomic anyway (never for the deterministic modes)
-        a.kchunk = k;
-        int split = 1;
-        if (mode == GEMM_ATOMIC && ctas < 2L * sms && k >= 128) {
-            const int bk = GemmK<T>::BK;
-            split = (int)std::min<long>(std::min<long>((2L * sms + ctas - 1) / ctas, 8), k / 64);
-            a.kchunk = ((k + split - 1) / split + bk - 1) / bk * bk;
-            split = (k + a.kchunk - 1) / a.kchunk;
-        }
-        dim3 grid((unsigned)nt, (unsigned)((m + bm - 1) / bm), (unsigned)split);
-        if (bm == 128) grouped_gemm_kernel<T, 128><<<grid, GM_THREADS, 0, s>>>(a);
-        else grouped_gemm_kernel<T, 64><<<grid, GM_THREADS, 0, s>>>(a);
-        TBEM_CK(cudaGetLastError());
-        if (launches) (*launches)++;
+    a.mode = mode;
+    a.kchunk = k;
+    const int nt = (int)it->second.first.n;
+    if (nt == 0) return;
+    const int bm = f64 ? DG_ROWS * DG_WARPS : gemm_bm(m);
+    const int mt = (m + bm - 1) / bm;
+    const long ctas = (long)nt * mt;
+    // split K when the tiles fill less than two CTAs per SM and the
+    // accumulation is atomic anyway (never for the deterministic modes)
+    int split = 1;
+    if (mode == GEMM_ATOMIC && ctas < 2L * sms && k >= 128) {
+        split = (int)std::min<long>(std::min<long>((2L * sms + ctas - 1) / ctas, 8), k / 64);
+        a.kchunk = ((k + split - 1) / split + GM_BK - 1) / GM_BK * GM_BK;
+        split = (k + a.kchunk - 1) / a.kchunk;
     }
+    const dim3 grid((unsigned)nt, (unsigned)mt, (unsigned)split);
+    if constexpr (f64) dgemm_warp_kernel<<<grid, 32 * DG_WARPS, 0, s>>>(a, bn);
+    else if (bm == 128) grouped_gemm_kernel<128><<<grid, GM_THREADS, 0, s>>>(a);
+    else grouped_gemm_kernel<64><<<grid, GM_THREADS, 0, s>>>(a);
+    TBEM_CK(cudaGetLastError());
+    if (launches) (*launches)++;
 }
 
-template void GemmSet::run_rect<double>(const double*, double*, int, int, int, int, int, int, cudaStream_t, long*, bool);
-template void GemmSet::run_rect<float>(const float*, float*, int, int, int, int, int, int, cudaStream_t, long*, bool);
+template void GemmSet::run_rect<double>(const double*, double*, int, int, int, int, int, int, cudaStream_t, long*);
+template void GemmSet::run_rect<float>(const float*, float*, int, int, int, int, int, int, cudaStream_t, long*);
 
 
 namespace {
@@ -231,9 +217,18 @@ __global__ void slot_reduce_kernel(const double* slots, const int* tgt, const in
     const long len = (long)nrhs * m;
     const int b = ptr[t], e = ptr[t + 1];
     double* d = D + (long)tgt[t] * len;
+    constexpr int U = 8;  // slots in flight per thread (added in order)
     for (long j = threadIdx.x; j < len; j += blockDim.x) {
         double acc = 0.0;
-        for (int q = b; q < e; q++) acc += slots[(long)idx[q] * len + j];
+        int q = b;
+        for (; q + U <= e; q += U) {
+            double v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) v[u] = slots[(long)idx[q + u] * len + j];
+#pragma unroll
+            for (int u = 0; u < U; u++) acc += v[u];
+        }
+        for (; q < e; q++) acc += slots[(long)idx[q] * len + j];
         d[j] += acc;
     }
 }
@@ -258,9 +253,11 @@ void SlotPlan::build(const GemmSet& G, long cap, const void* pool, size_t esz)
             idx.push_back(out_slot[i].second);
         }
         ptr.push_back((int)idx.size());
-        c.tgt.upload(tgt);
-        c.ptr.upload(ptr);
-        c.idx.upload(idx);
+        const size_t ot = c.table.add(tgt), op = c.table.add(ptr), oi = c.table.add(idx);
+        c.table.upload();
+        c.tgt = c.table.at<int>(ot);
+        c.ptr = c.table.at<int>(op);
+        c.idx = c.table.at<int>(oi);
         c.n_tgt = (int)tgt.size();
         c.gemm.upload(pool, esz);
         max_slots = std::max(max_slots, (long)idx.size());
@@ -296,7 +293,7 @@ void SlotPlan::run(const double* B, double* D, int m, int nrhs, int trans, doubl
     for (Chunk& c : chunks) {
         c.gemm.run_rect<double>(B, slots, m, m, m, nrhs, trans, GEMM_STORE, s, launches);
         if (c.n_tgt > 0) {
-            slot_reduce_kernel<<<c.n_tgt, 256, 0, s>>>(slots, c.tgt.p, c.ptr.p, c.idx.p, m, nrhs, D);
+            slot_reduce_kernel<<<c.n_tgt, 256, 0, s>>>(slots, c.tgt, c.ptr, c.idx, m, nrhs, D);
             TBEM_CK(cudaGetLastError());
             if (launches) (*launches)++;
         }
@@ -970,6 +967,15 @@ void Plan::autotune_tc()
     for (auto& g : f.l2l) { g.tc_bn = best_bn; g.tc_bk = best_bk; }
 }
 
+namespace {
+// A timed variant replaces the best one so far only when it is clearly faster:
+// near ties (variants within about 1 % on a 100 us pass, where repeated
+// timings differ by as much) would otherwise fall either way from one
+// construction to the next, and with them the summation order, which the plain
+// form's pseudo-inverses turn into 1e-8 of the result.
+constexpr float AUTOTUNE_MARGIN = 0.97f;
+}  // namespace
+
 // Picks the point-to-point pass's threads per target (2, 4 or 8) by timing
 // each variant on this operator's own task lists (zero densities: the cost
 // does not depend on the values).
@@ -986,8 +992,8 @@ void Plan::autotune_p2p()
     int best_tpt = 4;
     for (int tpt : {4, 2, 8}) {
         p2p_tpt = tpt;
-        float ms = 0.f;
-        for (int rep = 0; rep < 3; rep++) {
+        float ms = 1e30f;
+        for (int rep = 0; rep < 4; rep++) {
             TBEM_CK(cudaEventRecord(e0, stream));
             if (mixed)
                 eval<float>(p2p_set(), kid, false, false, otree, dobs, 0, *dsrc, 0, s32.p, n_src,
@@ -999,9 +1005,9 @@ void Plan::autotune_p2p()
             TBEM_CK(cudaEventSynchronize(e1));
             float t = 0.f;
             TBEM_CK(cudaEventElapsedTime(&t, e0, e1));
-            if (rep > 0) ms += t;  // the first run warms the caches
+            if (rep > 0) ms = std::min(ms, t);  // the first run warms the caches
         }
-        if (ms < best) {
+        if (ms < AUTOTUNE_MARGIN * best) {
             best = ms;
             best_tpt = tpt;
         }
@@ -1024,8 +1030,8 @@ void Plan::autotune_p2m()
     int best_tpt = 4;
     for (int tpt : {4, 2, 1}) {
         p2m_tpt = tpt;
-        float ms = 0.f;
-        for (int rep = 0; rep < 3; rep++) {
+        float ms = 1e30f;
+        for (int rep = 0; rep < 4; rep++) {
             TBEM_CK(cudaEventRecord(e0, stream));
             if (mixed)
                 eval<float>(p2m_set(), f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s32.p, n_src,
@@ -1037,9 +1043,9 @@ void Plan::autotune_p2m()
             TBEM_CK(cudaEventSynchronize(e1));
             float t = 0.f;
             TBEM_CK(cudaEventElapsedTime(&t, e0, e1));
-            if (rep > 0) ms += t;
+            if (rep > 0) ms = std::min(ms, t);
         }
-        if (ms < best) {
+        if (ms < AUTOTUNE_MARGIN * best) {
             best = ms;
             best_tpt = tpt;
         }
@@ -1624,17 +1630,30 @@ void Plan::build_gemm_sets(Form& F, long, long, long, const std::vector<long>& m
     }
     const void* pool = F.mixed ? (const void*)F.ops32.p : (const void*)F.ops64.p;
     const size_t esz = F.mixed ? sizeof(float) : sizeof(double);
-    for (auto& g : F.m2m) g.upload(pool, esz);
     for (auto& g : F.m2m_t) g.upload(pool, esz);
     for (auto& g : F.l2l) g.upload(pool, esz);
-    for (auto& g : F.l2l_t) g.upload(pool, esz);
-    F.m2l.upload(pool, esz);
-    F.m2l_t.upload(pool, esz);
-    if (!F.mixed) {
-        // the plain form's M2L through slots, at most ~1 GB of slots per RHS
+    if (F.mixed) {
+        for (auto& g : F.m2m) g.upload(pool, esz);
+        for (auto& g : F.l2l_t) g.upload(pool, esz);
+        F.m2l.upload(pool, esz);
+        F.m2l_t.upload(pool, esz);
+    } else {
+        // the plain form's M2L (and the sums over a parent's children, M2M and
+        // the transposed L2L) through slots, at most ~1 GB of slots per RHS
         const long cap = std::max<long>(1, (1L << 30) / (8L * n));
         F.m2l_slots.build(F.m2l, cap, pool, esz);
         F.m2l_t_slots.build(F.m2l_t, cap, pool, esz);
+        F.max_slots = std::max(F.m2l_slots.max_slots, F.m2l_t_slots.max_slots);
+        auto per_level = [&](std::vector<SlotPlan>& v, const std::vector<GemmSet>& sets) {
+            v.clear();
+            v.resize(sets.size());
+            for (size_t l = 0; l < sets.size(); l++) {
+                v[l].build(sets[l], cap, pool, esz);
+                F.max_slots = std::max(F.max_slots, v[l].max_slots);
+            }
+        };
+        per_level(F.m2m_slots, F.m2m);
+        per_level(F.l2l_t_slots, F.l2l_t);
     }
     // check-to-equivalent products, one group per level (FP64 pool)
     F.c2e_up.clear();
@@ -2371,8 +2390,7 @@ void Plan::ensure_rhs(int nrhs)
         qu64.ensure((size_t)ncs * nrhs * n);
         cd64.ensure((size_t)nco * nrhs * n);
         qd64.ensure((size_t)nco * nrhs * n);
-        const long slots = std::max(f.m2l_slots.max_slots, f.m2l_t_slots.max_slots);
-        if (slots > 0) slots64.ensure((size_t)slots * nrhs * n);
+        if (f.max_slots > 0) slots64.ensure((size_t)f.max_slots * nrhs * n);
     }
     cap_rhs = nrhs;
 }
@@ -2530,14 +2548,21 @@ void Plan::forward(int nrhs, cudaStream_t s)
         TBEM_CK(cudaMemsetAsync(cu64.p, 0, sizeof(double) * ncs * nrhs * n, s));
         TBEM_CK(cudaMemsetAsync(cd64.p, 0, sizeof(double) * nco * nrhs * n, s));
         mark("gather", s);
+        // the near field on the side stream: it fills the SMs that the upward
+        // pass, a chain of small launches, leaves idle
+        TBEM_CK(cudaEventRecord(ev_fork, s));
+        TBEM_CK(cudaStreamWaitEvent(side, ev_fork, 0));
+        eval<double>(p2p_set(), kid, false, false, O, dobs, 0, *dsrc, 0, s64.p, NS, nullptr, y64.p, NO, nullptr, 1, nrhs, side, false);
+        TBEM_CK(cudaEventRecord(ev_join, side));
         eval<double>(p2m_set(), F.ks_kid, true, false, S, *dsrc, F.r_uc, *dsrc, 0, s64.p, NS, nullptr, nullptr, 0, cu64.p, 0, nrhs, s, false);
         mark("p2m", s);
         for (int l = S.n_levels() - 1; l >= 0; l--) {
-            if (l < (int)F.m2m.size()) F.m2m[l].run<double>(qu64.p, cu64.p, n, nrhs, 0, GEMM_WAVES, s, &launches);
+            if (l < (int)F.m2m.size()) F.m2m_slots[l].run(qu64.p, cu64.p, n, nrhs, 0, slots64.p, s, &launches);
             F.c2e_up[l].run<double>(cu64.p, qu64.p, n, nrhs, 0, GEMM_STORE, s, &launches);
         }
         mark("m2m+c2e_up", s);
-        eval<double>(p2p_set(), kid, false, false, O, dobs, 0, *dsrc, 0, s64.p, NS, nullptr, y64.p, NO, nullptr, 1, nrhs, s, false);
+        // join the near field: the passes below add into the same outputs
+        TBEM_CK(cudaStreamWaitEvent(s, ev_join, 0));
         mark("p2p", s);
         eval<double>(m2p, F.kt_kid, false, true, O, dobs, 0, *dsrc, F.r_ue, nullptr, 0, qu64.p, y64.p, NO, nullptr, 1, nrhs, s, false);
         eval<double>(p2l, F.ks_kid, true, false, O, dobs, F.r_dc, *dsrc, 0, s64.p, NS, nullptr, nullptr, 0, cd64.p, 1, nrhs, s, false);
@@ -2654,7 +2679,7 @@ void Plan::adjoint(int nrhs, cudaStream_t s)
         // down pass reversed: deepest level first
         for (int l = O.n_levels() - 1; l >= 0; l--) {
             F.c2e_dn_t[l].run<double>(qd64.p, cd64.p, n, nrhs, 1, GEMM_STORE, s, &launches);
-            if (l > 0 && l - 1 < (int)F.l2l_t.size()) F.l2l_t[l - 1].run<double>(cd64.p, qd64.p, n, nrhs, 1, GEMM_WAVES, s, &launches);
+            if (l > 0 && l - 1 < (int)F.l2l_t.size()) F.l2l_t_slots[l - 1].run(cd64.p, qd64.p, n, nrhs, 1, slots64.p, s, &launches);
         }
         if (F.m2l_on_the_fly)
             eval<double>(m2l_fly_t, F.g_kid, true, true, S, *dsrc, F.r_ue, dobs, F.r_dc, nullptr, 0, cd64.p, nullptr, 0, qu64.p, 1, nrhs, s, true);
@@ -2933,7 +2958,7 @@ int Plan::rhs_chunk(int nrhs) const
         if (!L.m2p.empty() || f.m2l_on_the_fly) per += 8.0 * (2 * ncs + nco) * n;
     } else {
         per += 8.0 * 2 * (ncs + nco) * n;
-        per += 8.0 * std::max(f.m2l_slots.max_slots, f.m2l_t_slots.max_slots) * n;
+        per += 8.0 * f.max_slots * n;
     }
     return (int)std::max<double>(1.0, std::min<double>(nrhs, std::floor(RHS_WORK_BUDGET / per)));
 }

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <cusolverDn.h>
 
+#include <cstring>
 #include <map>
 #include <memory>
 #include <tuple>
@@ -140,6 +141,29 @@ struct DBuf {
     }
 };
 
+// Several host arrays in one device allocation (each 16-byte aligned), copied
+// in with one transfer: a construction makes hundreds of small index tables,
+// and an allocation, a copy and a wait for each are what their upload costs.
+struct PackedTable {
+    DBuf<char> buf;
+    std::vector<char> host;
+    template <typename T>
+    size_t add(const std::vector<T>& v)
+    {
+        const size_t off = host.size();
+        host.resize(off + (v.size() * sizeof(T) + 15) / 16 * 16);
+        if (!v.empty()) std::memcpy(host.data() + off, v.data(), v.size() * sizeof(T));
+        return off;
+    }
+    void upload()
+    {
+        buf.upload(host.data(), host.size());
+        host = std::vector<char>();
+    }
+    template <typename T>
+    const T* at(size_t off) const { return reinterpret_cast<const T*>(buf.p + off); }
+};
+
 // A timing event destroyed on every exit path (the autotuners time
 // candidates between two of these).
 struct ScopedEvent {
@@ -211,15 +235,12 @@ struct GemmSet {
     std::vector<long> pair0;
     std::vector<int> npairs;
     std::vector<int> in_cell, out_cell;
-    DBuf<long> d_pair0;
-    DBuf<int> d_npairs, d_in, d_out;
-    DBuf<const void*> d_A;  // resolved pointers
-    std::map<int, std::pair<DBuf<int>, DBuf<int>>> tiles;  // per nrhs
-    // conflict-free waves for GEMM_WAVES (built on first use)
-    std::vector<int> wave_of;
-    int n_waves = 0;
-    std::map<int, std::vector<int>> wave_tile_start;  // per nrhs: first tile of every wave
-    void build_waves();
+    // device copies (one allocation); d_A: resolved operator pointers
+    PackedTable table;
+    const long* d_pair0 = nullptr;
+    const int *d_npairs = nullptr, *d_in = nullptr, *d_out = nullptr;
+    const void* const* d_A = nullptr;
+    std::map<std::pair<int, int>, std::pair<DBuf<int>, DBuf<int>>> tiles;  // per (nrhs, tile columns)
     long total_pairs() const { return (long)in_cell.size(); }
     bool empty() const { return in_cell.empty(); }
     void add_group(long a_off, const std::vector<std::pair<int, int>>& pairs);
@@ -233,7 +254,7 @@ struct GemmSet {
     // op(A) is m x k; A is stored row-major with rows of length lda
     template <typename T>
     void run_rect(const T* B, T* D, int m, int k, int lda, int nrhs, int trans, int mode,
-                  cudaStream_t s, long* launches = nullptr, bool tables_only = false);
+                  cudaStream_t s, long* launches = nullptr);
     // tensor-core path (B taken from P's split planes; D columns of P.m rows);
     // nn = elements per operator in the pool the groups' offsets refer to
     struct TcTiles {
@@ -250,7 +271,8 @@ struct GemmSet {
 
 // Deterministic accumulation of a GEMM set whose groups add into the same
 // outputs (the plain form's M2L: every observation cell receives one product
-// per source of its interaction list).  Every pair's product is stored in a
+// per source of its interaction list; its M2M and transposed L2L: one per
+// child).  Every pair's product is stored in a
 // slot of its own -- one GEMM launch over all groups, [slot][rhs][m] -- and
 // each output column then sums its slots in pair order: a fixed summation
 // order with no atomics and two launches per chunk.  The pairs run in chunks
@@ -258,7 +280,9 @@ struct GemmSet {
 struct SlotPlan {
     struct Chunk {
         GemmSet gemm;             // the chunk's groups, out_cell = local slot
-        DBuf<int> tgt, ptr, idx;  // output cells with slots, CSR of their local slots
+        // output cells with slots, CSR of their local slots
+        PackedTable table;
+        const int *tgt = nullptr, *ptr = nullptr, *idx = nullptr;
         int n_tgt = 0;
     };
     std::vector<Chunk> chunks;
@@ -292,8 +316,10 @@ struct Form {
     DBuf<float> ops32;                          // mixed: combined M2M', L2L', U_k
     std::vector<GemmSet> c2e_up, m2m, l2l, c2e_dn;  // per level
     GemmSet m2l;
-    // plain form: the M2L products through slots (deterministic, no waves)
+    // plain form: the products that meet in one output through slots
     SlotPlan m2l_slots, m2l_t_slots;
+    std::vector<SlotPlan> m2m_slots, l2l_t_slots;  // per level
+    long max_slots = 0;
     // transposed sets (in/out swapped) for the adjoint apply
     std::vector<GemmSet> c2e_up_t, m2m_t, l2l_t, c2e_dn_t;
     GemmSet m2l_t;

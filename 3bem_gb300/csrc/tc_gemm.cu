@@ -576,8 +576,8 @@ void GemmSet::run_tc(const TcPlanes& P, float* D, int nrhs, int atomic, long nn,
     a.tiles = it->second.t.p;
     a.tile_brow = it->second.brow.p;
     a.tile_drow = it->second.drow.p;
-    a.in_cell = d_in.p;
-    a.out_cell = d_out.p;
+    a.in_cell = d_in;
+    a.out_cell = d_out;
     a.nrhs = nrhs;
     a.D = D;
     a.n = P.m;
