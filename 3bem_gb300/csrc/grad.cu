@@ -2,98 +2,134 @@
 // with respect to every point position, normal and weight, and to x (the
 // direct operator's transpose apply), in FP64.
 //
-// The kernel tensors are differentiated exactly by forward-mode dual numbers:
-// kernel_tensor<T> (kernels.cuh) is evaluated with T = Dual<3> seeded on the
-// separation delta = y - x (d/dy = d/ddelta, d/dx = -d/ddelta), on the source
-// normal, or on the observation normal.  Two passes, each owning its outputs
-// (no atomics): a source-owner pass (gradients of y_j, n_j, w_j and x_j) and
-// an observation-owner pass (gradients of x_i and n_i).  Direct O(N M) sums:
-// the workload this serves (24,576 sources x 16,384 observers) takes a
-// fraction of a second.
+// The contraction c = rho^T K(d; no, ns) chi of every kernel is a rational
+// function of d, its length and a few dot products, so its derivatives in the
+// separation d = y - x (d/dy = d/dd, d/dx = -d/dd) and in the normals are
+// written out (grad_pair) in the powers of 1 / |d| that the value needs
+// anyway.  The direct passes each own their outputs (no atomics): a
+// source-owner pass (gradients of y_j, n_j, w_j and x_j) and an
+// observation-owner pass (gradients of x_i and n_i), O(N M) sums.
 #include <string>
+#include <type_traits>
 
 #include "plan.h"
 
 namespace tbem {
 namespace {
 
-struct Dual3 {
-    double v, g[3];
-    __device__ Dual3() : v(0), g{0, 0, 0} {}
-    __device__ Dual3(double x) : v(x), g{0, 0, 0} {}
-};
-__device__ __forceinline__ Dual3 operator+(const Dual3& a, const Dual3& b)
+// Which derivatives of one pair are wanted besides the value.
+enum GradNormal { GN_NONE = 0, GN_SRC = 1, GN_OBS = 2 };
+
+// The normal a kernel's value depends on, as seen from one side: the normals'
+// derivatives are taken at the target of the pass only.
+__host__ __device__ constexpr bool grad_src_normal(int kid) { return kid == LAP_D || kid == EL_TRAC || kid == EL_HYP; }
+__host__ __device__ constexpr bool grad_obs_normal(int kid) { return kid == EL_ADJ || kid == EL_HYP; }
+
+__device__ __forceinline__ double dot3(const double* a, const double* b)
 {
-    Dual3 r; r.v = a.v + b.v;
-    for (int k = 0; k < 3; k++) r.g[k] = a.g[k] + b.g[k];
-    return r;
-}
-__device__ __forceinline__ Dual3 operator-(const Dual3& a, const Dual3& b)
-{
-    Dual3 r; r.v = a.v - b.v;
-    for (int k = 0; k < 3; k++) r.g[k] = a.g[k] - b.g[k];
-    return r;
-}
-__device__ __forceinline__ Dual3 operator-(const Dual3& a)
-{
-    Dual3 r; r.v = -a.v;
-    for (int k = 0; k < 3; k++) r.g[k] = -a.g[k];
-    return r;
-}
-__device__ __forceinline__ Dual3 operator*(const Dual3& a, const Dual3& b)
-{
-    Dual3 r; r.v = a.v * b.v;
-    for (int k = 0; k < 3; k++) r.g[k] = a.g[k] * b.v + a.v * b.g[k];
-    return r;
-}
-__device__ __forceinline__ Dual3 operator/(const Dual3& a, const Dual3& b)
-{
-    Dual3 r; r.v = a.v / b.v;
-    const double ib = 1.0 / b.v;
-    for (int k = 0; k < 3; k++) r.g[k] = (a.g[k] - r.v * b.g[k]) * ib;
-    return r;
-}
-__device__ __forceinline__ bool operator<(const Dual3& a, const Dual3& b) { return a.v < b.v; }
-__device__ __forceinline__ Dual3 sqrt(const Dual3& a)
-{
-    Dual3 r; r.v = ::sqrt(a.v);
-    const double h = r.v > 0 ? 0.5 / r.v : 0.0;
-    for (int k = 0; k < 3; k++) r.g[k] = a.g[k] * h;
-    return r;
+    return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
 }
 
-// which: 0 seeds delta, 1 the source normal, 2 the observation normal
-__device__ __forceinline__ Dual3 contraction(int kid, int which, const double* d, const double* no,
-                                            const double* ns, const double* rv, const double* xv,
-                                            const KParams& p)
+// c = rho^T K(d; m, n) chi without the kernel's leading constant (m the
+// observation normal, n the source normal), its gradient gd in d and gn in
+// the source (WN = GN_SRC) or observation (GN_OBS) normal, by the formulas of
+// kernels.cuh:
+//   displacement  c = q (c2 rho.chi + a b q^2),  q = 1 / |d|, a = rho.d, b = chi.d
+//   traction / adjoint traction, w their normal, g = w.d, s = -1 / +1:
+//     c = s q^3 (c2 rho.chi g + 3 a b g q^2 + s c2 (w.chi a - w.rho b))
+//   hypersingular, h = n.d, g = m.d:
+//     c = q^3 C0 + 3 q^5 Q - 15 q^7 a b g h
+// Zero for the self pair.
+template <int KID, int WN>
+__device__ __forceinline__ void grad_pair(const double* d, const double* m, const double* n, const double* rho,
+                                          const double* chi, double c2, double& c, double* gd, double* gn)
 {
-    Dual3 D[3], NO[3], NS[3];
-    for (int k = 0; k < 3; k++) {
-        D[k] = Dual3(d[k]);
-        NO[k] = Dual3(no[k]);
-        NS[k] = Dual3(ns[k]);
+    c = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) gd[k] = gn[k] = 0;
+    const double r2 = dot3(d, d);
+    if (r2 < 1e-12) return;
+    if constexpr (KID == IDENT) {
+        c = rho[0] * chi[0];
+        return;
     }
-    Dual3* seed = which == 0 ? D : which == 1 ? NS : NO;
-    for (int k = 0; k < 3; k++) seed[k].g[k] = 1.0;
-    Dual3 K[9];
-    kernel_tensor<Dual3>(kid, D[0], D[1], D[2], NO[0], NO[1], NO[2], NS[0], NS[1], NS[2], p, K);
-    const int R = kernel_dim(kid);
-    Dual3 c(0.0);
-    for (int a = 0; a < R; a++)
-        for (int b = 0; b < R; b++) c = c + K[a * R + b] * Dual3(rv[a] * xv[b]);
-    return c;
+    const double q = rsqrt(r2), q2 = q * q, q3 = q2 * q;
+    if constexpr (KID == LAP_S) {
+        c = rho[0] * chi[0] * q;
+        const double f = -c * q2;
+#pragma unroll
+        for (int k = 0; k < 3; k++) gd[k] = f * d[k];
+    } else if constexpr (KID == LAP_D) {
+        const double f = rho[0] * chi[0] * q3;
+        c = f * dot3(n, d);
+        const double e = -3.0 * c * q2;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            gd[k] = f * n[k] + e * d[k];
+            if (WN == GN_SRC) gn[k] = f * d[k];
+        }
+    } else if constexpr (KID == EL_DISP) {
+        const double a = dot3(rho, d), b = dot3(chi, d), P = c2 * dot3(rho, chi);
+        const double t = a * b * q2;
+        c = q * (P + t);
+        const double e = -q3 * (P + 3.0 * t), fa = q3 * a, fb = q3 * b;
+#pragma unroll
+        for (int k = 0; k < 3; k++) gd[k] = e * d[k] + fb * rho[k] + fa * chi[k];
+    } else if constexpr (KID == EL_TRAC || KID == EL_ADJ) {
+        const double sg = KID == EL_TRAC ? -1.0 : 1.0;
+        const double* w = KID == EL_TRAC ? n : m;
+        const double a = dot3(rho, d), b = dot3(chi, d), g = dot3(w, d);
+        const double wc = sg * c2 * dot3(w, chi), wr = sg * c2 * dot3(w, rho);
+        const double P = c2 * dot3(rho, chi), t = 3.0 * a * b * q2;
+        const double f = sg * q3;
+        const double u = P + t;
+        const double N = u * g + wc * a - wr * b;
+        c = f * N;
+        const double g3 = 3.0 * g * q2;
+        const double er = f * (g3 * b + wc), ec = f * (g3 * a - wr), ew = f * u;
+        const double ed = -f * q2 * (3.0 * N + 2.0 * t * g);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            gd[k] = er * rho[k] + ec * chi[k] + ew * w[k] + ed * d[k];
+            if (WN != GN_NONE) gn[k] = f * (u * d[k] + sg * c2 * (a * chi[k] - b * rho[k]));
+        }
+    } else {
+        const double nu = 0.5 * (1.0 - c2), c4 = 4.0 * nu - 1.0;
+        const double a = dot3(rho, d), b = dot3(chi, d), g = dot3(m, d), h = dot3(n, d);
+        const double rm = dot3(rho, m), rn = dot3(rho, n), xm = dot3(chi, m), xn = dot3(chi, n);
+        const double rx = dot3(rho, chi), nm = dot3(n, m);
+        const double C0 = c2 * (rx * nm + rn * xm) + c4 * xn * rm;
+        const double Q = c2 * (rm * b * h + xn * a * g) + nu * (xm * a * h + rx * g * h + rn * b * g + nm * a * b);
+        const double q5 = q3 * q2, q7 = q5 * q2, ab = a * b, gh = g * h;
+        c = q3 * C0 + 3.0 * q5 * Q - 15.0 * q7 * ab * gh;
+        const double ed = -3.0 * q5 * C0 - 15.0 * q7 * Q + 105.0 * q7 * q2 * ab * gh;
+        const double er = 3.0 * q5 * (nu * (xm * h + nm * b) + c2 * xn * g) - 15.0 * q7 * b * gh;
+        const double ec = 3.0 * q5 * (nu * (rn * g + nm * a) + c2 * rm * h) - 15.0 * q7 * a * gh;
+        const double em = 3.0 * q5 * (nu * (rx * h + rn * b) + c2 * xn * a) - 15.0 * q7 * ab * h;
+        const double en = 3.0 * q5 * (nu * (xm * a + rx * g) + c2 * rm * b) - 15.0 * q7 * ab * g;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            gd[k] = ed * d[k] + er * rho[k] + ec * chi[k] + em * m[k] + en * n[k];
+            if (WN == GN_SRC)
+                gn[k] = q3 * (c2 * (rx * m[k] + xm * rho[k]) + c4 * rm * chi[k]) + en * d[k] +
+                        3.0 * q5 * (c2 * a * g * chi[k] + nu * (b * g * rho[k] + ab * m[k]));
+            if (WN == GN_OBS)
+                gn[k] = q3 * (c2 * (rx * n[k] + rn * chi[k]) + c4 * xn * rho[k]) + em * d[k] +
+                        3.0 * q5 * (c2 * b * h * rho[k] + nu * (a * h * chi[k] + ab * n[k]));
+        }
+    }
 }
 
 // Source owner: g_y, g_ns, g_w, g_x (= A^T r) for source j.
-__global__ void grad_src_kernel(int kid, KParams p, const double* ox, const double* on, long n_obs,
+template <int KID>
+__global__ void grad_src_kernel(KParams p, const double* ox, const double* on, long n_obs,
                                 const double* sx, const double* sn, const double* sw, long n_src,
                                 const double* x, const double* r, double* g_y, double* g_ns,
                                 double* g_w, double* g_x)
 {
     const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n_src) return;
-    const int R = kernel_dim(kid);
-    const bool use_ns = kid == LAP_D || kid == EL_TRAC || kid == EL_HYP;
+    constexpr int R = kernel_dim(KID);
     double xv[3] = {0, 0, 0};
     for (int b = 0; b < R; b++) xv[b] = x[b * n_src + j];
     const double y[3] = {sx[3 * j], sx[3 * j + 1], sx[3 * j + 2]};
@@ -104,38 +140,34 @@ __global__ void grad_src_kernel(int kid, KParams p, const double* ox, const doub
         const double noi[3] = {on[3 * i], on[3 * i + 1], on[3 * i + 2]};
         double rv[3] = {0, 0, 0};
         for (int a = 0; a < R; a++) rv[a] = r[a * n_obs + i];
-        const Dual3 c = contraction(kid, 0, d, noi, nsj, rv, xv, p);
-        gw += c.v;
-        for (int k = 0; k < 3; k++) gy[k] += c.g[k];
-        if (use_ns) {
-            const Dual3 cn = contraction(kid, 1, d, noi, nsj, rv, xv, p);
-            for (int k = 0; k < 3; k++) gn[k] += cn.g[k];
+        double c, gd[3], g2[3];
+        grad_pair<KID, grad_src_normal(KID) ? GN_SRC : GN_NONE>(d, noi, nsj, rv, xv, p.c2, c, gd, g2);
+        gw += c;
+        for (int k = 0; k < 3; k++) {
+            gy[k] += gd[k];
+            gn[k] += g2[k];
         }
-        // x gradient: sum_a r_a K_ab, i.e. the contraction with x = e_b
-        double K[9];
-        kernel_tensor<double>(kid, d[0], d[1], d[2], noi[0], noi[1], noi[2], nsj[0], nsj[1], nsj[2], p, K);
-        for (int b = 0; b < R; b++)
-            for (int a = 0; a < R; a++) gx[b] += rv[a] * K[a * R + b];
+        accumulate<KID, true, double>(d[0], d[1], d[2], noi[0], noi[1], noi[2], nsj[0], nsj[1], nsj[2], p.c2, rv, gx);
     }
-    const double w = sw[j];
+    const double w = sw[j] * p.scale;
     for (int k = 0; k < 3; k++) {
         if (g_y) g_y[3 * j + k] = w * gy[k];
         if (g_ns) g_ns[3 * j + k] = w * gn[k];
     }
-    if (g_w) g_w[j] = gw;
+    if (g_w) g_w[j] = p.scale * gw;
     if (g_x)
         for (int b = 0; b < R; b++) g_x[b * n_src + j] = w * gx[b];
 }
 
-// Observation owner: g_x_obs (= -dL/ddelta summed) and g_no for observer i.
-__global__ void grad_obs_kernel(int kid, KParams p, const double* ox, const double* on, long n_obs,
+// Observation owner: g_x_obs (= -dL/dd summed) and g_no for observer i.
+template <int KID>
+__global__ void grad_obs_kernel(KParams p, const double* ox, const double* on, long n_obs,
                                 const double* sx, const double* sn, const double* sw, long n_src,
                                 const double* x, const double* r, double* g_o, double* g_no)
 {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_obs) return;
-    const int R = kernel_dim(kid);
-    const bool use_no = kid == EL_ADJ || kid == EL_HYP;
+    constexpr int R = kernel_dim(KID);
     double rv[3] = {0, 0, 0};
     for (int a = 0; a < R; a++) rv[a] = r[a * n_obs + i];
     const double o[3] = {ox[3 * i], ox[3 * i + 1], ox[3 * i + 2]};
@@ -146,16 +178,32 @@ __global__ void grad_obs_kernel(int kid, KParams p, const double* ox, const doub
         const double nsj[3] = {sn[3 * j], sn[3 * j + 1], sn[3 * j + 2]};
         double xv[3] = {0, 0, 0};
         for (int b = 0; b < R; b++) xv[b] = sw[j] * x[b * n_src + j];
-        const Dual3 c = contraction(kid, 0, d, noi, nsj, rv, xv, p);
-        for (int k = 0; k < 3; k++) go[k] -= c.g[k];
-        if (use_no) {
-            const Dual3 cn = contraction(kid, 2, d, noi, nsj, rv, xv, p);
-            for (int k = 0; k < 3; k++) gn[k] += cn.g[k];
+        double c, gd[3], g2[3];
+        grad_pair<KID, grad_obs_normal(KID) ? GN_OBS : GN_NONE>(d, noi, nsj, rv, xv, p.c2, c, gd, g2);
+        for (int k = 0; k < 3; k++) {
+            go[k] -= gd[k];
+            gn[k] += g2[k];
         }
     }
     for (int k = 0; k < 3; k++) {
-        if (g_o) g_o[3 * i + k] = go[k];
-        if (g_no) g_no[3 * i + k] = gn[k];
+        if (g_o) g_o[3 * i + k] = p.scale * go[k];
+        if (g_no) g_no[3 * i + k] = p.scale * gn[k];
+    }
+}
+
+// f(std::integral_constant<int, KID>) for a 3D kernel id
+template <typename F>
+void with_kernel(int kid, F&& f)
+{
+    switch (kid) {
+    case LAP_S: f(std::integral_constant<int, LAP_S>()); break;
+    case LAP_D: f(std::integral_constant<int, LAP_D>()); break;
+    case EL_DISP: f(std::integral_constant<int, EL_DISP>()); break;
+    case EL_TRAC: f(std::integral_constant<int, EL_TRAC>()); break;
+    case EL_ADJ: f(std::integral_constant<int, EL_ADJ>()); break;
+    case EL_HYP: f(std::integral_constant<int, EL_HYP>()); break;
+    case IDENT: f(std::integral_constant<int, IDENT>()); break;
+    default: throw Error(TBEM_ERR_ARG, "gradients take the 3D kernels");
     }
 }
 
@@ -165,9 +213,13 @@ __global__ void grad_obs_kernel(int kid, KParams p, const double* ox, const doub
 // surface with the transposed state as its density (P2M^T, P2L^T) -- the
 // contraction c = v(z)^T K(y_j - z; n_z, n_j) x_j, its gradient in y_j and
 // (kernels with a source normal) in n_j are summed; the sums of c are
-// dL/dw_j.  GRAD_TPT threads per target split its sources and meet in warp
-// shuffles; the work items are those of the transposed task sets (32
-// targets per CTA of 128 threads).
+// dL/dw_j.  The pass is paced by the FP64 pipe (two FMAs per SM and clock, 40
+// to 110 of them per pair), so what matters is that every SM has pairs: the
+// transposed task sets' work items (32 targets) are cut into GRAD_SUB CTAs of
+// eight targets each, GRAD_TPT threads per target split its sources and meet
+// in warp shuffles.  With one CTA of four threads per target per item and
+// forward-mode dual numbers through the kernel tensors, the four passes of
+// 6,144 sources and 4,096 observers took 28.4 ms in 107 to 182 CTAs; now 2.5 ms.
 struct GradEvalArgs {
     const int* item_task;
     const int* item_start;
@@ -193,82 +245,98 @@ struct GradEvalArgs {
     const double* q64;
     int kid;
     KParams kp;
-    int want_n;
     // 0: the targets are the operator's source points (contraction v^T K x_j,
     // derivatives in y_j and n_j); 1: its observation points (r_i^T K v,
     // derivatives in x_i and the observation normal n_i)
     int obs_side;
     double* g;             // [t_n][7]: d/dposition (3), d/dnormal (3), value (1); accumulated
 };
-constexpr int GRAD_TPT = 4, GRAD_THREADS = 128;
+constexpr int GRAD_TPT = 16, GRAD_THREADS = 128;
+constexpr int GRAD_TARGETS = GRAD_THREADS / GRAD_TPT;           // targets per CTA
+constexpr int GRAD_SUB = (EVAL_THREADS / 4) / GRAD_TARGETS;     // CTAs per work item
 
-template <bool SRC_SURF>
+template <int KID, bool OBS_SIDE, bool SRC_SURF>
 __global__ void __launch_bounds__(GRAD_THREADS) grad_eval_kernel(const GradEvalArgs a)
 {
+    constexpr int R = kernel_dim(KID);
+    constexpr int WN = OBS_SIDE ? (grad_obs_normal(KID) ? GN_OBS : GN_NONE) : (grad_src_normal(KID) ? GN_SRC : GN_NONE);
+    constexpr bool NORMALS = normal_dot_kernel(KID);  // the kernel's value depends on a normal
     const int task = a.item_task[blockIdx.x];
-    const int ti = a.item_start[blockIdx.x] + (int)threadIdx.x / GRAD_TPT;
+    const int ti = a.item_start[blockIdx.x] + (int)(blockIdx.y * GRAD_TARGETS + threadIdx.x / GRAD_TPT);
     const int lane = threadIdx.x % GRAD_TPT;
     const bool active = ti < a.task_tgt_count[task];
-    const int R = kernel_dim(a.kid);
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     if (active) {
         const long j = a.task_tgt[task] + ti;
         const double y[3] = {a.t_xyz[3 * j], a.t_xyz[3 * j + 1], a.t_xyz[3 * j + 2]};
-        const double nj[3] = {a.t_nrm[3 * j], a.t_nrm[3 * j + 1], a.t_nrm[3 * j + 2]};
+        double nj[3] = {0, 0, 0};
+        if (NORMALS)
+            for (int k = 0; k < 3; k++) nj[k] = a.t_nrm[3 * j + k];
         double xv[3] = {0, 0, 0};
+#pragma unroll
         for (int b = 0; b < R; b++) xv[b] = a.t_x[b * a.t_n + j];
         for (int blk = a.task_src_ptr[task]; blk < a.task_src_ptr[task + 1]; blk++) {
             const long sb = a.src_blk[blk];
             const int cnt = a.src_blk_count[blk];
+            // a surface's points are c + t u: y - z = (y - c) - t u
+            double yc[3] = {0, 0, 0}, t = 0;
+            if (SRC_SURF) {
+                t = a.s_rad[sb] * a.s_rref;
+#pragma unroll
+                for (int k = 0; k < 3; k++) yc[k] = y[k] - a.s_center[3 * sb + k];
+            }
             for (int li = lane; li < cnt; li += GRAD_TPT) {
-                double z[3], nz[3], rv[3] = {0, 0, 0};
+                double dd[3], nz[3] = {0, 0, 0}, rv[3] = {0, 0, 0};
                 if (SRC_SURF) {
-                    const double rr = a.s_rad[sb];
+#pragma unroll
                     for (int k = 0; k < 3; k++) {
                         const double u = a.unit[3 * li + k];
-                        z[k] = rr * (a.s_rref * u) + a.s_center[3 * sb + k];
-                        nz[k] = u;
+                        dd[k] = fma(-t, u, yc[k]);
+                        if (NORMALS) nz[k] = u;
                     }
                     const long base = sb * (long)(R * a.ns) + li;
+#pragma unroll
                     for (int d = 0; d < R; d++)
                         rv[d] = a.q32 ? (double)a.q32[base + d * a.ns] : a.q64[base + d * a.ns];
                 } else {
                     const long p = sb + li;
+#pragma unroll
                     for (int k = 0; k < 3; k++) {
-                        z[k] = a.s_xyz[3 * p + k];
-                        nz[k] = a.s_nrm[3 * p + k];
+                        dd[k] = y[k] - a.s_xyz[3 * p + k];
+                        if (NORMALS) nz[k] = a.s_nrm[3 * p + k];
                     }
+#pragma unroll
                     for (int d = 0; d < R; d++) rv[d] = a.s_v[d * a.s_n + p];
                 }
-                if (!a.obs_side) {
+                double c, gd[3], gn[3];
+                if (!OBS_SIDE) {
                     // forward separation y_j - z, the target the source side
-                    const double dd[3] = {y[0] - z[0], y[1] - z[1], y[2] - z[2]};
-                    const Dual3 c = contraction(a.kid, 0, dd, nz, nj, rv, xv, a.kp);
-                    acc[6] += c.v;
-                    for (int k = 0; k < 3; k++) acc[k] += c.g[k];
-                    if (a.want_n) {
-                        const Dual3 cn = contraction(a.kid, 1, dd, nz, nj, rv, xv, a.kp);
-                        for (int k = 0; k < 3; k++) acc[3 + k] += cn.g[k];
-                    }
+                    grad_pair<KID, WN>(dd, nz, nj, rv, xv, a.kp.c2, c, gd, gn);
+                    acc[6] += c;
+#pragma unroll
+                    for (int k = 0; k < 3; k++) acc[k] += gd[k];
                 } else {
                     // forward separation z - x_i: d/dx_i = -d/dd
-                    const double dd[3] = {z[0] - y[0], z[1] - y[1], z[2] - y[2]};
-                    const Dual3 c = contraction(a.kid, 0, dd, nj, nz, xv, rv, a.kp);
-                    acc[6] += c.v;
-                    for (int k = 0; k < 3; k++) acc[k] -= c.g[k];
-                    if (a.want_n) {
-                        const Dual3 cn = contraction(a.kid, 2, dd, nj, nz, xv, rv, a.kp);
-                        for (int k = 0; k < 3; k++) acc[3 + k] += cn.g[k];
-                    }
+                    const double df[3] = {-dd[0], -dd[1], -dd[2]};
+                    grad_pair<KID, WN>(df, nj, nz, xv, rv, a.kp.c2, c, gd, gn);
+#pragma unroll
+                    for (int k = 0; k < 3; k++) acc[k] -= gd[k];
+                }
+                if (WN != GN_NONE) {
+#pragma unroll
+                    for (int k = 0; k < 3; k++) acc[3 + k] += gn[k];
                 }
             }
         }
     }
+#pragma unroll
     for (int off = GRAD_TPT / 2; off > 0; off /= 2)
+#pragma unroll
         for (int i = 0; i < 7; i++) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
     if (!active || lane != 0) return;
     double* g = a.g + 7 * (a.task_tgt[task] + ti);
-    for (int i = 0; i < 7; i++) g[i] += acc[i];
+#pragma unroll
+    for (int i = 0; i < 7; i++) g[i] += a.kp.scale * acc[i];
 }
 
 // Tree order [n][7] -> the caller's order: g_y = w dL/dy, g_n = w dL/dn,
@@ -341,8 +409,17 @@ void grad_pass(const TaskSet& ts, bool src_surf, GradEvalArgs a, cudaStream_t s,
     a.task_src_ptr = ts.d_src_ptr.p;
     a.src_blk = ts.d_blk.p;
     a.src_blk_count = ts.d_blk_count.p;
-    if (src_surf) grad_eval_kernel<true><<<ts.n_items(), GRAD_THREADS, 0, s>>>(a);
-    else grad_eval_kernel<false><<<ts.n_items(), GRAD_THREADS, 0, s>>>(a);
+    const dim3 grid((unsigned)ts.n_items(), GRAD_SUB);
+    with_kernel(a.kid, [&](auto K) {
+        constexpr int kid = decltype(K)::value;
+        if (a.obs_side) {
+            if (src_surf) grad_eval_kernel<kid, true, true><<<grid, GRAD_THREADS, 0, s>>>(a);
+            else grad_eval_kernel<kid, true, false><<<grid, GRAD_THREADS, 0, s>>>(a);
+        } else {
+            if (src_surf) grad_eval_kernel<kid, false, true><<<grid, GRAD_THREADS, 0, s>>>(a);
+            else grad_eval_kernel<kid, false, false><<<grid, GRAD_THREADS, 0, s>>>(a);
+        }
+    });
     TBEM_CK(cudaGetLastError());
     if (launches) (*launches)++;
 }
@@ -419,11 +496,9 @@ void Plan::source_gradients(const double* x, const double* r, double* g_y, doubl
     a.unit = d_unit.p;
     a.ns = ns;
     a.g = g7;
-    auto with_normals = [](int k) { return k == LAP_D || k == EL_TRAC || k == EL_HYP; };
     // P2P^T: the observation points with the densities r
     a.kid = kid;
     a.kp = make_kparams(kid, mu, nu);
-    a.want_n = with_normals(kid);
     a.s_xyz = dobs.xyz.p;
     a.s_nrm = dobs.nrm64.p;
     a.s_v = rt;
@@ -432,7 +507,6 @@ void Plan::source_gradients(const double* x, const double* r, double* g_y, doubl
     // P2M^T and P2L^T: check surfaces with the transposed states
     a.kid = f.ks_kid;
     a.kp = make_kparams(f.ks_kid, mu, nu);
-    a.want_n = with_normals(f.ks_kid);
     a.q32 = f.f64 ? nullptr : cu32.p;
     a.q64 = f.f64 ? cu64.p : nullptr;
     a.s_center = dsrc->center.p;
@@ -538,11 +612,9 @@ void Plan::observation_gradients(const double* x, const double* r, double* g_x, 
     a.unit = d_unit.p;
     a.ns = ns;
     a.g = g7;
-    auto with_obs_normals = [](int k) { return k == EL_ADJ || k == EL_HYP; };
     // P2P: the source points with densities w x
     a.kid = kid;
     a.kp = make_kparams(kid, mu, nu);
-    a.want_n = with_obs_normals(kid);
     a.s_xyz = dsrc->xyz.p;
     a.s_nrm = dsrc->nrm64.p;
     a.s_v = xt;
@@ -551,7 +623,6 @@ void Plan::observation_gradients(const double* x, const double* r, double* g_x, 
     // M2P and L2P: equivalent surfaces, the kernel that reaches the targets
     a.kid = f.kt_kid;
     a.kp = make_kparams(f.kt_kid, mu, nu);
-    a.want_n = with_obs_normals(f.kt_kid);
     if (!L.m2p.empty()) {
         a.q32 = nullptr;
         a.q64 = f.f64 ? cu64.p : qu64.p;
@@ -612,9 +683,10 @@ extern "C" int tbem_direct_gradients(int kernel, const double* kernel_params,
                 for (Out* o : {&gs, &gns, &gw, &gx})
                     if (o->p) TBEM_CK(cudaMemsetAsync(o->p, 0, o->n * sizeof(double), s));
             } else {
-                grad_src_kernel<<<(unsigned)((n_src + 127) / 128), 128, 0, s>>>(
-                    kernel, kp, ol.p, on.p, n_obs, sl.p, sn.p, sw.p, n_src, xs.p, rs.p, gs.p, gns.p,
-                    gw.p, gx.p);
+                with_kernel(kernel, [&](auto K) {
+                    grad_src_kernel<decltype(K)::value><<<(unsigned)((n_src + 127) / 128), 128, 0, s>>>(
+                        kp, ol.p, on.p, n_obs, sl.p, sn.p, sw.p, n_src, xs.p, rs.p, gs.p, gns.p, gw.p, gx.p);
+                });
                 TBEM_CK(cudaGetLastError());
             }
         }
@@ -623,8 +695,10 @@ extern "C" int tbem_direct_gradients(int kernel, const double* kernel_params,
                 for (Out* o : {&go, &gno})
                     if (o->p) TBEM_CK(cudaMemsetAsync(o->p, 0, o->n * sizeof(double), s));
             } else {
-                grad_obs_kernel<<<(unsigned)((n_obs + 127) / 128), 128, 0, s>>>(
-                    kernel, kp, ol.p, on.p, n_obs, sl.p, sn.p, sw.p, n_src, xs.p, rs.p, go.p, gno.p);
+                with_kernel(kernel, [&](auto K) {
+                    grad_obs_kernel<decltype(K)::value><<<(unsigned)((n_obs + 127) / 128), 128, 0, s>>>(
+                        kp, ol.p, on.p, n_obs, sl.p, sn.p, sw.p, n_src, xs.p, rs.p, go.p, gno.p);
+                });
                 TBEM_CK(cudaGetLastError());
             }
         }
