@@ -3,6 +3,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "handle.h"
@@ -69,45 +70,101 @@ __global__ void weight_kernel(const double* x, const double* w, double* s, long 
 
 // y = A x (add = 0) or y += A x (add = 1).  L lanes per row (L chosen per
 // matrix from its mean row length): a lane takes the row's entries k = b +
-// lane, + L, ..., CSR_UNROLL of them per step, loading all their values and
-// columns before any gather of x, so every lane keeps CSR_UNROLL independent
-// loads in flight (the gather x[col[k]] waits on the column load: with one
-// entry per lane per step the SpMV was latency-bound at a third of the
-// copy bandwidth); the L partial sums meet in shuffles.
-constexpr int CSR_UNROLL = 4, CSR_THREADS = 256;
+// lane, + L, ..., CSR_UNROLL of them per step, and the L partial sums meet in
+// shuffles.  HBM-bound: 12 bytes per entry (FP64 value, 32-bit column; 64-bit
+// columns only where there are 2^31 of them).
+constexpr int CSR_UNROLL = 4, CSR_THREADS = 256, CSR_CTAS_PER_SM = 4, CSR_RHS = 4;
 
-template <int L>
-__global__ void __launch_bounds__(CSR_THREADS)
-csr_kernel(const long* __restrict__ rowptr, const long* __restrict__ col, const double* __restrict__ val,
-           const double* __restrict__ x, double* y, long n_rows, long n_cols, int nrhs, int add)
+// The step of the row ending at entry e that starts at entry b: this lane's
+// values and columns (-1 past the end), all loads independent.
+template <int L, typename I>
+__device__ __forceinline__ void csr_step(const double* val, const I* col, long b, long e, int lane,
+                                         double (&v)[CSR_UNROLL], I (&c)[CSR_UNROLL])
 {
-    const long row = ((long)blockIdx.x * blockDim.x + threadIdx.x) / L;
+    const int n = (int)min(e - b, (long)CSR_UNROLL * L);
+    const double* pv = val + b + lane;
+    const I* pc = col + b + lane;
+#pragma unroll
+    for (int u = 0; u < CSR_UNROLL; u++) {
+        const bool in = lane + u * L < n;
+        v[u] = in ? __ldg(pv + u * L) : 0.0;
+        c[u] = in ? __ldg(pc + u * L) : I(-1);
+    }
+}
+
+// NR right-hand sides (up to CSR_RHS; the entries are read once for all of
+// them).  Two things pace it besides HBM.  The FP64 pipe takes
+// 16 clocks per warp instruction, so the L-lane sums matter: a row of 50
+// entries on 16 lanes is 4 FMA and 4 shuffle additions for two rows, on 4
+// lanes 13 and 2 for eight.  And a row is three dependent reads (row start,
+// entries, gather of x), so a thread that lived for one row would have its
+// entry loads in flight a third of the time: the CTAs that fit the chip walk
+// the rows, a warp's 32 / L rows in step, and load the next step -- of these
+// rows, or the first of the warp's next ones, whose row starts are read one
+// set ahead -- before they gather for the current one.  184,320
+// rows of 50 entries (110 MB): 61 us with one row per 16-lane group and 64-bit
+// columns, 33 us now; deeper or shallower steps and other occupancies (2 to 8
+// entries, 3 to 8 CTAs per SM) measured within 3 % of that.
+template <int L, int NR, typename I>
+__global__ void __launch_bounds__(CSR_THREADS, NR == 1 ? CSR_CTAS_PER_SM : CSR_CTAS_PER_SM - 1)
+csr_kernel(const long* __restrict__ rowptr, const I* __restrict__ col, const double* __restrict__ val,
+           const double* __restrict__ x, double* y, long n_rows, long n_cols, int add)
+{
+    constexpr int U = CSR_UNROLL;
     const int lane = threadIdx.x % L;
-    if (row >= n_rows) return;  // whole L-lane groups leave together
-    const unsigned mask = L == 32 ? 0xffffffffu : (((1u << L) - 1u) << ((threadIdx.x % 32) / L * L));
-    const long b = rowptr[row], e = rowptr[row + 1];
-    for (int r = 0; r < nrhs; r++) {
-        const double* xr = x + (long)r * n_cols;
-        double acc = 0.0;
-        for (long k0 = b + lane; k0 < e; k0 += (long)CSR_UNROLL * L) {
-            double v[CSR_UNROLL];
-            long c[CSR_UNROLL];
+    const long stride = (long)gridDim.x * (CSR_THREADS / L);
+    long row = (long)blockIdx.x * (CSR_THREADS / L) + threadIdx.x / L;
+    const long row0 = row - (threadIdx.x % 32) / L;  // the warp's first row
+    double v[U], v2[U];
+    I c[U], c2[U];
+    // rows past the end have no entries
+    auto bounds = [&](long r, long& rb, long& re) {
+        rb = r < n_rows ? rowptr[r] : 0;
+        re = r < n_rows ? rowptr[r + 1] : 0;
+    };
+    long b, e, nb, ne;
+    bounds(row, b, e);
+    bounds(row + stride, nb, ne);
+    csr_step<L>(val, col, b, e, lane, v, c);
+    for (long set = row0; set < n_rows; set += stride) {
+        long nnb, nne;
+        bounds(row + 2 * stride, nnb, nne);
+        // steps of the longest of the warp's rows
+        const long mine = (e - b + U * L - 1) / (U * L);
+        const int steps = (int)max(1u, __reduce_max_sync(0xffffffffu, (unsigned)min(mine, (long)INT32_MAX)));
+        double acc[NR];
 #pragma unroll
-            for (int u = 0; u < CSR_UNROLL; u++) {
-                const long k = k0 + (long)u * L;
-                v[u] = k < e ? val[k] : 0.0;
-                c[u] = k < e ? col[k] : -1;
+        for (int r = 0; r < NR; r++) acc[r] = 0.0;
+        for (int st = 1; st <= steps; st++) {
+            b += U * L;
+            if (st < steps) csr_step<L>(val, col, min(b, e), e, lane, v2, c2);
+            else csr_step<L>(val, col, nb, ne, lane, v2, c2);
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (c[u] >= 0) {
+#pragma unroll
+                    for (int r = 0; r < NR; r++) acc[r] += v[u] * x[r * n_cols + c[u]];
+                }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                v[u] = v2[u];
+                c[u] = c2[u];
             }
-#pragma unroll
-            for (int u = 0; u < CSR_UNROLL; u++)
-                if (c[u] >= 0) acc += v[u] * xr[c[u]];
         }
 #pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(mask, acc, o);
-        if (lane == 0) {
-            double* d = y + (long)r * n_rows + row;
-            *d = add ? *d + acc : acc;
+        for (int r = 0; r < NR; r++) {
+#pragma unroll
+            for (int o = L / 2; o > 0; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+            if (lane == 0 && row < n_rows) {
+                double* d = y + r * n_rows + row;
+                *d = add ? *d + acc[r] : acc[r];
+            }
         }
+        row += stride;
+        b = nb;
+        e = ne;
+        nb = nnb;
+        ne = nne;
     }
 }
 
@@ -177,7 +234,9 @@ double fma_peak(int device)
 struct TbemCsr {
     long n_rows = 0, n_cols = 0, nnz = 0;
     int lanes = 32;  // lanes per row of the SpMV kernel
-    tbem::DBuf<long> rowptr, col;
+    tbem::DBuf<long> rowptr;
+    tbem::DBuf<int> col;        // n_cols <= 2^31 - 1
+    tbem::DBuf<long> col_wide;  // else
     tbem::DBuf<double> val;
 };
 
@@ -186,15 +245,36 @@ namespace {
 void csr_launch(const TbemCsr* A, const double* x, double* y, int nrhs, int add, cudaStream_t s)
 {
     const int L = A->lanes;
-    const unsigned blocks = (unsigned)((A->n_rows * L + CSR_THREADS - 1) / CSR_THREADS);
-    auto go = [&](auto kern) {
-        kern<<<blocks, CSR_THREADS, 0, s>>>(A->rowptr.p, A->col.p, A->val.p, x, y, A->n_rows, A->n_cols,
-                                            nrhs, add);
+    int dev = 0, sms = 0;
+    TBEM_CK(cudaGetDevice(&dev));
+    TBEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const long need = (A->n_rows * L + CSR_THREADS - 1) / CSR_THREADS;
+    const unsigned blocks = (unsigned)std::min<long>(need, (long)CSR_CTAS_PER_SM * std::max(sms, 1));
+    auto with_lanes = [&](auto lanes, const auto* col) {
+        constexpr int LL = decltype(lanes)::value;
+        for (int r0 = 0; r0 < nrhs; r0 += CSR_RHS) {
+            const double* xr = x + (long)r0 * A->n_cols;
+            double* yr = y + (long)r0 * A->n_rows;
+            auto launch = [&](auto kern) {
+                kern<<<blocks, CSR_THREADS, 0, s>>>(A->rowptr.p, col, A->val.p, xr, yr, A->n_rows, A->n_cols, add);
+            };
+            using I = std::remove_const_t<std::remove_pointer_t<decltype(col)>>;
+            switch (std::min(nrhs - r0, CSR_RHS)) {
+            case 1: launch(csr_kernel<LL, 1, I>); break;
+            case 2: launch(csr_kernel<LL, 2, I>); break;
+            case 3: launch(csr_kernel<LL, 3, I>); break;
+            default: launch(csr_kernel<LL, 4, I>);
+            }
+        }
     };
-    if (L == 4) go(csr_kernel<4>);
-    else if (L == 8) go(csr_kernel<8>);
-    else if (L == 16) go(csr_kernel<16>);
-    else go(csr_kernel<32>);
+    auto go = [&](const auto* col) {
+        if (L == 4) with_lanes(std::integral_constant<int, 4>(), col);
+        else if (L == 8) with_lanes(std::integral_constant<int, 8>(), col);
+        else if (L == 16) with_lanes(std::integral_constant<int, 16>(), col);
+        else with_lanes(std::integral_constant<int, 32>(), col);
+    };
+    if (A->col.p) go(A->col.p);
+    else go(A->col_wide.p);
     TBEM_CK(cudaGetLastError());
 }
 }  // namespace
@@ -288,14 +368,18 @@ int tbem_csr_create(long n_rows, long n_cols, const double* values, const long* 
             if (row_ptrs[i + 1] < row_ptrs[i]) throw Error(TBEM_ERR_ARG, "row_ptrs must not decrease");
         const long nnz = row_ptrs[n_rows];
         if (nnz > 0 && (!values || !column_indices)) throw Error(TBEM_ERR_ARG, "null values");
-        // column check on all host cores, in blocks (one flag per block)
+        // column check (and narrowing) on all host cores, in blocks (one flag per block)
+        const bool wide = n_cols > (long)INT32_MAX;
+        std::vector<int> narrow(wide ? 0 : nnz);
         const long block = 1 << 20, n_blocks = (nnz + block - 1) / block;
         std::vector<char> bad(n_blocks, 0);
         nf::parallel_for(
             n_blocks,
             [&](long b) {
-                for (long k = b * block; k < std::min(nnz, (b + 1) * block); k++)
+                for (long k = b * block; k < std::min(nnz, (b + 1) * block); k++) {
                     if (column_indices[k] < 0 || column_indices[k] >= n_cols) bad[b] = 1;
+                    if (!wide) narrow[k] = (int)column_indices[k];
+                }
             },
             1);
         if (std::find(bad.begin(), bad.end(), 1) != bad.end())
@@ -305,11 +389,15 @@ int tbem_csr_create(long n_rows, long n_cols, const double* values, const long* 
         h->n_cols = n_cols;
         h->nnz = nnz;
         // lanes per row: the fewest that take a mean row in one unrolled step
+        // (its latency), but no more than give the chip a thousand threads
+        // per SM: from there on fewer lanes add less on the FP64 pipe
         const double mean = n_rows > 0 ? (double)nnz / (double)n_rows : 0.0;
         h->lanes = mean <= 4 * CSR_UNROLL ? 4 : mean <= 8 * CSR_UNROLL ? 8 : mean <= 16 * CSR_UNROLL ? 16 : 32;
+        while (h->lanes > 4 && n_rows * (h->lanes / 2) >= 152L * 1024) h->lanes /= 2;
         h->rowptr.upload(row_ptrs, (size_t)n_rows + 1);
         if (nnz > 0) {
-            h->col.upload(column_indices, (size_t)nnz);
+            if (wide) h->col_wide.upload(column_indices, (size_t)nnz);
+            else h->col.upload(narrow);
             h->val.upload(values, (size_t)nnz);
         }
         *out = h.release();
@@ -368,8 +456,15 @@ int tbem_csr_download(const TbemCsr* h, double* values, long* column_indices, lo
             TBEM_CK(cudaMemcpy(row_ptrs, h->rowptr.p, sizeof(long) * (h->n_rows + 1), cudaMemcpyDeviceToHost));
         if (h->nnz > 0 && values)
             TBEM_CK(cudaMemcpy(values, h->val.p, sizeof(double) * h->nnz, cudaMemcpyDeviceToHost));
-        if (h->nnz > 0 && column_indices)
-            TBEM_CK(cudaMemcpy(column_indices, h->col.p, sizeof(long) * h->nnz, cudaMemcpyDeviceToHost));
+        if (h->nnz > 0 && column_indices) {
+            if (h->col.p) {
+                std::vector<int> narrow(h->nnz);
+                TBEM_CK(cudaMemcpy(narrow.data(), h->col.p, sizeof(int) * h->nnz, cudaMemcpyDeviceToHost));
+                std::copy(narrow.begin(), narrow.end(), column_indices);
+            } else {
+                TBEM_CK(cudaMemcpy(column_indices, h->col_wide.p, sizeof(long) * h->nnz, cudaMemcpyDeviceToHost));
+            }
+        }
         return TBEM_OK;
     } catch (...) {
         return tbem::api_status();
