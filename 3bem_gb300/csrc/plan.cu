@@ -17,6 +17,7 @@
 #include <mutex>
 #include <numeric>
 #include <tuple>
+#include <type_traits>
 
 #include "nearfield.h"
 #include "plan.h"
@@ -579,22 +580,72 @@ __global__ void __launch_bounds__(256) l2p_mixed_kernel(const float* E, const lo
     }
 }
 
-// Its transpose: cd[leaf][r][k] = sum_rows E[row][k] z[r][d][pt0 + i].
-template <typename T>
-__global__ void l2p_mixed_t_kernel(const T* E, const long* row0, const int* leaf,
-                                   const long* pt0, const int* npts, const T* z, long z_n,
-                                   int n, int ld, int R, int nrhs, T* cd)
+// Its transpose: cd[leaf][r][k] = sum_rows E[row][k] z[r][d][pt0 + i], for NR
+// right-hand sides from r0.  HBM-bound on E: one CTA per leaf reads whole rows
+// in 16-byte pieces, a thread per piece of the row and as many row groups as
+// the CTA holds, four rows in flight per thread; the leaf's inputs sit in
+// shared memory and the row groups' sums meet there in a fixed order.  24,576
+// points, r_out 256 (E 78 MB): 45 us with a thread per column and a row at a
+// time, 27 us now.
+constexpr int L2PT_THREADS = 256, L2PT_ROWS = 128;
+template <typename T, int NR>
+__global__ void __launch_bounds__(L2PT_THREADS) l2p_mixed_t_kernel(
+    const T* E, const long* row0, const int* leaf, const long* pt0, const int* npts, const T* z, long z_n,
+    int n, int ld, int R, int nrhs, int r0, T* cd)
 {
+    constexpr int V = 16 / (int)sizeof(T);
+    using Vec = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+    __shared__ T zs[NR][L2PT_ROWS];
+    __shared__ T red[L2PT_THREADS * V];
     const int t = blockIdx.x;
     const int rows = npts[t] * R;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        for (int r = 0; r < nrhs; r++) {
-            T acc = 0;
-            for (int row = 0; row < rows; row++) {
-                const int i = row / R, d = row % R;
-                acc += E[(row0[t] + row) * (long)ld + k] * z[((long)r * R + d) * z_n + pt0[t] + i];
+    const T* Et = E + row0[t] * (long)ld;
+    const int Q = (n + V - 1) / V;  // pieces of a row (the padding beyond n is zero)
+    for (int qb = 0; qb < Q; qb += L2PT_THREADS) {
+        const int nq = min(Q - qb, L2PT_THREADS), G = L2PT_THREADS / nq;
+        const int q = threadIdx.x % nq, g = threadIdx.x / nq;
+        T acc[NR][V];
+#pragma unroll
+        for (int r = 0; r < NR; r++)
+#pragma unroll
+            for (int c = 0; c < V; c++) acc[r][c] = T(0);
+        for (int rt = 0; rt < rows; rt += L2PT_ROWS) {
+            const int nr = min(rows - rt, L2PT_ROWS);
+            __syncthreads();
+            for (int e = threadIdx.x; e < nr * NR; e += L2PT_THREADS) {
+                const int r = e / nr, row = rt + e % nr;
+                zs[r][e % nr] = r0 + r < nrhs ? z[((long)(r0 + r) * R + row % R) * z_n + pt0[t] + row / R] : T(0);
             }
-            cd[((long)leaf[t] * nrhs + r) * n + k] = acc;
+            __syncthreads();
+            if (g >= G) continue;
+            const T* Eq = Et + (long)rt * ld + (qb + q) * V;
+#pragma unroll 4
+            for (int row = g; row < nr; row += G) {
+                const Vec w = __ldcs(reinterpret_cast<const Vec*>(Eq + (long)row * ld));
+                T v[V];
+                if constexpr (sizeof(T) == 4) { v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w; }
+                else { v[0] = w.x; v[1] = w.y; }
+#pragma unroll
+                for (int r = 0; r < NR; r++)
+#pragma unroll
+                    for (int c = 0; c < V; c++) acc[r][c] += v[c] * zs[r][row];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            __syncthreads();
+            if (g < G)
+#pragma unroll
+                for (int c = 0; c < V; c++) red[(g * nq + q) * V + c] = acc[r][c];
+            __syncthreads();
+            if (r0 + r < nrhs)
+                for (int e = threadIdx.x; e < nq * V; e += L2PT_THREADS) {
+                    const int k = qb * V + e;
+                    if (k >= n) continue;
+                    T v = T(0);
+                    for (int gg = 0; gg < G; gg++) v += red[gg * nq * V + e];
+                    cd[((long)leaf[t] * nrhs + r0 + r) * n + k] = v;
+                }
         }
     }
 }
@@ -963,6 +1014,8 @@ void Plan::autotune_tc()
     }
     G.tc_bn = best_bn;
     G.tc_bk = best_bk;
+    f.m2l_c_t.tc_bn = best_bn;
+    f.m2l_c_t.tc_bk = best_bk;
     for (auto& g : f.m2m) { g.tc_bn = best_bn; g.tc_bk = best_bk; }
     for (auto& g : f.l2l) { g.tc_bn = best_bn; g.tc_bk = best_bk; }
 }
@@ -2424,6 +2477,25 @@ void Plan::launch_l2p(const T* cd, int len, int nrhs, cudaStream_t s)
     launches++;
 }
 
+// The transposed L2P of `nrhs` right-hand sides z ([rhs][R][n_obs]) into the
+// leaves' states cd ([cell][rhs][len]): four right-hand sides per pass over E.
+template <typename T>
+void Plan::launch_l2p_t(const T* z, int len, int nrhs, T* cd, cudaStream_t s)
+{
+    Form& F = f;
+    const T* E;
+    if constexpr (sizeof(T) == 4) E = F.E.p; else E = F.E64.p;
+    for (int r0 = 0; r0 < nrhs;) {
+        const bool one = nrhs - r0 == 1;
+        auto kern = one ? l2p_mixed_t_kernel<T, 1> : l2p_mixed_t_kernel<T, 4>;
+        kern<<<F.n_l2p, L2PT_THREADS, 0, s>>>(E, F.E_row0.p, F.E_leaf.p, F.E_pt0.p, F.E_npts.p, z, n_obs, len,
+                                              F.E_ld, R, nrhs, r0, cd);
+        TBEM_CK(cudaGetLastError());
+        launches++;
+        r0 += one ? 1 : 4;
+    }
+}
+
 void Plan::mark(const char* name, cudaStream_t s)
 {
     if (!timing) return;
@@ -2675,7 +2747,12 @@ void Plan::adjoint(int nrhs, cudaStream_t s)
         // L2P^T, M2P^T, P2P^T
         eval<double>(l2p_t, F.kt_kid, true, false, O, dobs, F.r_de, dobs, 0, y64.p, NO, nullptr, nullptr, 0, qd64.p, 1, nrhs, s, true);
         eval<double>(m2p_t, F.kt_kid, true, false, S, *dsrc, F.r_ue, dobs, 0, y64.p, NO, nullptr, nullptr, 0, qu64.p, 1, nrhs, s, true);
-        eval<double>(p2p_t, kid, false, false, S, *dsrc, 0, dobs, 0, y64.p, NO, nullptr, s64.p, NS, nullptr, 1, nrhs, s, true);
+        // the near field on the side stream, joined before the passes that add
+        // into the same outputs
+        TBEM_CK(cudaEventRecord(ev_fork, s));
+        TBEM_CK(cudaStreamWaitEvent(side, ev_fork, 0));
+        eval<double>(p2p_t, kid, false, false, S, *dsrc, 0, dobs, 0, y64.p, NO, nullptr, s64.p, NS, nullptr, 1, nrhs, side, true);
+        TBEM_CK(cudaEventRecord(ev_join, side));
         // down pass reversed: deepest level first
         for (int l = O.n_levels() - 1; l >= 0; l--) {
             F.c2e_dn_t[l].run<double>(qd64.p, cd64.p, n, nrhs, 1, GEMM_STORE, s, &launches);
@@ -2685,6 +2762,7 @@ void Plan::adjoint(int nrhs, cudaStream_t s)
             eval<double>(m2l_fly_t, F.g_kid, true, true, S, *dsrc, F.r_ue, dobs, F.r_dc, nullptr, 0, cd64.p, nullptr, 0, qu64.p, 1, nrhs, s, true);
         else
             F.m2l_t_slots.run(cd64.p, qu64.p, n, nrhs, 1, slots64.p, s, &launches);
+        TBEM_CK(cudaStreamWaitEvent(s, ev_join, 0));
         eval<double>(p2l_t, F.ks_kid, false, true, S, *dsrc, 0, dobs, F.r_dc, nullptr, 0, cd64.p, s64.p, NS, nullptr, 1, nrhs, s, true);
         // up pass reversed: root first
         for (int l = 0; l < S.n_levels(); l++) {
@@ -2699,9 +2777,7 @@ void Plan::adjoint(int nrhs, cudaStream_t s)
         TBEM_CK(cudaMemsetAsync(cu32.p, 0, sizeof(float) * ncs * nrhs * n, s));
         TBEM_CK(cudaMemsetAsync(cd32.p, 0, sizeof(float) * nco * nrhs * n, s));
         if (F.n_l2p > 0) {
-            l2p_mixed_t_kernel<float><<<F.n_l2p, 256, 0, s>>>(F.E.p, F.E_row0.p, F.E_leaf.p, F.E_pt0.p, F.E_npts.p, s32.p, NO, n, F.E_ld, R, nrhs, cd32.p);
-            TBEM_CK(cudaGetLastError());
-            launches++;
+            launch_l2p_t(s32.p, n, nrhs, cd32.p, s);
         }
         eval<float>(p2p_t, kid, false, false, S, *dsrc, 0, dobs, 0, s32.p, NO, nullptr, s64.p, NS, nullptr, 1, nrhs, s, true);
         const bool need64 = !L.m2p.empty() || F.m2l_on_the_fly;
@@ -2844,24 +2920,40 @@ void Plan::adjoint_compressed(int nrhs, cudaStream_t s)
     T* cd = pick<T>(cd32, cd64);
     T* cuc = pick<T>(cuc32, cuc64);
     T* cdc = pick<T>(cdc32, cdc64);
-    const T* E;
-    if constexpr (sizeof(T) == 4) E = F.E.p; else E = F.E64.p;
     gather_kernel<T><<<grid_for(NO * R * nrhs), 256, 0, s>>>(xin, dobs.perm.p, nullptr, zin, NO, R, nrhs);
     TBEM_CK(cudaGetLastError());
     launches++;
     TBEM_CK(cudaMemsetAsync(cuc, 0, sizeof(T) * ncs * nrhs * ri, s));
     TBEM_CK(cudaMemsetAsync(cdc, 0, sizeof(T) * nco * nrhs * ro, s));
+    // the near field on the side stream, as in the forward apply
+    TBEM_CK(cudaEventRecord(ev_fork, s));
+    TBEM_CK(cudaStreamWaitEvent(side, ev_fork, 0));
+    eval<T>(p2p_t, kid, false, false, S, *dsrc, 0, dobs, 0, zin, NO, nullptr, s64.p, NS, nullptr, 1, nrhs, side, true);
+    TBEM_CK(cudaEventRecord(ev_join, side));
+    bool joined = false;
+    auto join = [&] {  // before the passes that add into the same outputs
+        if (!joined) TBEM_CK(cudaStreamWaitEvent(s, ev_join, 0));
+        joined = true;
+    };
     if (F.n_l2p > 0) {
-        l2p_mixed_t_kernel<T><<<F.n_l2p, 256, 0, s>>>(E, F.E_row0.p, F.E_leaf.p, F.E_pt0.p, F.E_npts.p, zin, NO, ro, F.E_ld, R, nrhs, cdc);
-        TBEM_CK(cudaGetLastError());
-        launches++;
+        launch_l2p_t(zin, ro, nrhs, cdc, s);
     }
-    eval<T>(p2p_t, kid, false, false, S, *dsrc, 0, dobs, 0, zin, NO, nullptr, s64.p, NS, nullptr, 1, nrhs, s, true);
     for (int l = O.n_levels() - 1; l >= 1; l--)
         if (l - 1 < (int)F.l2l_c_t.size()) F.l2l_c_t[l - 1].run_rect<T>(cdc, cdc, ro, ro, ro, nrhs, 1, GEMM_ATOMIC, s, &launches);
-    F.m2l_c_t.run_rect<T>(cdc, cuc, ri, ro, ri, nrhs, 1, GEMM_ATOMIC, s, &launches);
+    // C_k^T on the tensor cores from the forward planes, as the forward M2L
+    bool tc_done = false;
+    if constexpr (sizeof(T) == 4) {
+        if (F.use_tc_c) {
+            F.tc_c.split_b_rows(cdc, 0, nco * nrhs, std::max(ncs, nco) * nrhs, s, true);
+            launches++;
+            F.m2l_c_t.run_tc(F.tc_c, cuc, nrhs, 1, (long)ro * ri, s, &launches, true);
+            tc_done = true;
+        }
+    }
+    if (!tc_done) F.m2l_c_t.run_rect<T>(cdc, cuc, ri, ro, ri, nrhs, 1, GEMM_ATOMIC, s, &launches);
     if (!L.p2l.empty()) {
         F.comp_p2l.run_rect<T>(cdc, cd, n, ro, ro, nrhs, 0, GEMM_STORE, s, &launches);
+        join();
         eval<T>(p2l_t, F.ks_kid, false, true, S, *dsrc, 0, dobs, F.r_dc, nullptr, 0, cd, s64.p, NS, nullptr, 1, nrhs, s, true);
     }
     if (!L.m2p.empty()) {
@@ -2891,6 +2983,7 @@ void Plan::adjoint_compressed(int nrhs, cudaStream_t s)
     // or an earlier apply's values)
     TBEM_CK(cudaMemsetAsync(cu, 0, sizeof(T) * ncs * nrhs * n, s));
     F.comp_p2m.run_rect<T>(cuc, cu, n, ri, n, nrhs, 1, GEMM_STORE, s, &launches);
+    join();
     eval<T>(p2m_t, F.ks_kid, false, true, S, *dsrc, 0, *dsrc, F.r_uc, nullptr, 0, cu, s64.p, NS, nullptr, 1, nrhs, s, true);
 }
 

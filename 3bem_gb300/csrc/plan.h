@@ -223,10 +223,11 @@ struct TcPlanes {
     DBuf<int> err;  // set by a tensor-core GEMM whose bounded wait gave up
     long long wait_cycles = 0;  // budget of the GEMM's bounded waits (0: the default)
     void build(const float* ops32, long n_ops, int m, int k, cudaStream_t s);
-    void split_b(const float* cells, long rows, cudaStream_t s);
-    // split only rows [row0, row0 + rows) of a [rows_total][k] buffer into
-    // the same rows of the planes (capacity for rows_total rows)
-    void split_b_rows(const float* cells, long row0, long rows, long rows_total, cudaStream_t s);
+    // split rows [row0, row0 + rows) of a [rows_total][k] buffer (trans: [m],
+    // the B operand of A^T) into the same rows of the planes (capacity for
+    // rows_total rows)
+    void split_b_rows(const float* cells, long row0, long rows, long rows_total, cudaStream_t s,
+                      bool trans = false);
 };
 
 // A set of GEMM groups (gemm.cuh) sharing B and D buffers.
@@ -265,8 +266,9 @@ struct GemmSet {
     std::map<int, TcTiles> tc_tiles;  // per (nrhs, N tile)
     int tc_bn = 128;  // N tile of the tensor-core path (128 or 64; autotuned)
     int tc_bk = 64;   // K chunk (64, or 32 with N = 128; autotuned)
+    // trans: op(A) = A^T (B from planes split with trans, D columns of P.k rows)
     void run_tc(const TcPlanes& P, float* D, int nrhs, int atomic, long nn, cudaStream_t s,
-                long* launches);
+                long* launches, bool trans = false);
 };
 
 // Deterministic accumulation of a GEMM set whose groups add into the same
@@ -520,6 +522,8 @@ struct Plan {
     void mark(const char* name, cudaStream_t s);
     template <typename T>
     void launch_l2p(const T* cd, int len, int nrhs, cudaStream_t s);
+    template <typename T>
+    void launch_l2p_t(const T* z, int len, int nrhs, T* cd, cudaStream_t s);
     size_t l2p_smem_set[2] = {0, 0};  // dynamic shared memory opted in for the many-RHS L2P (FP32, FP64)
     // operator pool layout of the current form
     std::vector<int> m2m_key_level, l2l_key_level;
