@@ -216,10 +216,9 @@ void with_kernel(int kid, F&& f)
 // dL/dw_j.  The pass is paced by the FP64 pipe (two FMAs per SM and clock, 40
 // to 110 of them per pair), so what matters is that every SM has pairs: the
 // transposed task sets' work items (32 targets) are cut into GRAD_SUB CTAs of
-// eight targets each, GRAD_TPT threads per target split its sources and meet
-// in warp shuffles.  With one CTA of four threads per target per item and
+// one warp per target, whose lanes split its sources and meet in shuffles.  With one CTA of four threads per target per item and
 // forward-mode dual numbers through the kernel tensors, the four passes of
-// 6,144 sources and 4,096 observers took 28.4 ms in 107 to 182 CTAs; now 2.5 ms.
+// 6,144 sources and 4,096 observers took 28.4 ms in 107 to 182 CTAs; now 2.3 ms.
 struct GradEvalArgs {
     const int* item_task;
     const int* item_start;
@@ -251,7 +250,7 @@ struct GradEvalArgs {
     int obs_side;
     double* g;             // [t_n][7]: d/dposition (3), d/dnormal (3), value (1); accumulated
 };
-constexpr int GRAD_TPT = 16, GRAD_THREADS = 128;
+constexpr int GRAD_TPT = 32, GRAD_THREADS = 128;
 constexpr int GRAD_TARGETS = GRAD_THREADS / GRAD_TPT;           // targets per CTA
 constexpr int GRAD_SUB = (EVAL_THREADS / 4) / GRAD_TARGETS;     // CTAs per work item
 
@@ -591,17 +590,8 @@ void Plan::observation_gradients(const double* x, const double* r, double* g_x, 
         widen_kernel<<<blocks_for(nco * n), 256, 0, s>>>(cd32.p, uck, nco * n);
         TBEM_CK(cudaGetLastError());
     }
-    TBEM_CKB(cublasSetStream(cublas, s));
-    const double one = 1.0, zero = 0.0;
-    for (int l = 0; l < O.n_levels() && l < (int)f.c2e_dn_off.size(); l++) {
-        const long c0 = O.level_start[l], c1 = O.level_start[l + 1];
-        if (c1 <= c0) continue;
-        // column-major q (n x cells) = C2E^T-as-stored^T u: the row-major
-        // pseudo-inverse applied to every cell's potential
-        TBEM_CKB(cublasDgemm(cublas, CUBLAS_OP_T, CUBLAS_OP_N, n, (int)(c1 - c0), n, &one,
-                             f.c2e.p + f.c2e_dn_off[l], n, uck + c0 * n, n, &zero, qdn + c0 * n, n));
-    }
-    TBEM_CKB(cublasSetStream(cublas, stream));
+    for (int l = 0; l < O.n_levels() && l < (int)f.c2e_l2p.size(); l++)
+        f.c2e_l2p[l].run<double>(uck, qdn, n, 1, 0, GEMM_STORE, s, &launches);
     TBEM_CK(cudaMemsetAsync(g7, 0, sizeof(double) * 7 * NO, s));
     GradEvalArgs a{};
     a.obs_side = 1;

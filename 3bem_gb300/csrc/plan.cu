@@ -2365,6 +2365,13 @@ void Plan::build_compression(Form& F, const CompressionInput& in)
         for (int c : L.l2p) a.push_back({c, c});
         F.decomp_l2p.add_group(0, a);
     }
+    F.c2e_l2p.clear();
+    F.c2e_l2p.resize(F.c2e_dn_off.size());
+    {
+        std::vector<std::vector<std::pair<int, int>>> a(F.c2e_l2p.size());
+        for (int c : L.l2p) a[O.cells[c].level].push_back({c, c});
+        for (size_t l = 0; l < a.size(); l++) F.c2e_l2p[l].add_group(F.c2e_dn_off[l], a[l]);
+    }
     // the sets resolve their operators in the pool of the form's precision
     const size_t es = f64 ? sizeof(double) : sizeof(float);
     auto pool = [&](DBuf<float>& p32, DBuf<double>& p64) -> const void* {
@@ -2380,6 +2387,7 @@ void Plan::build_compression(Form& F, const CompressionInput& in)
     F.decomp_m2p.upload(pool(F.Wl, F.Wl64), es);
     F.comp_p2l.upload(pool(F.Vb, F.Vb64), es);
     F.decomp_l2p.upload(pool(F.Vb, F.Vb64), es);
+    for (auto& g : F.c2e_l2p) g.upload(F.c2e.p, sizeof(double));
     F.m2l_compressed = true;
 }
 

@@ -354,6 +354,7 @@ struct Form {
     DBuf<double> V64;  // V in FP64 (column-major n x r_out) while the L2P operators are built
     GemmSet m2l_c, m2l_c_t, comp_p2m, decomp_m2p, comp_p2l;
     GemmSet decomp_l2p;  // V over the L2P leaves: their down-check potentials (gradients)
+    std::vector<GemmSet> c2e_l2p;  // per level: C2E_down over those leaves
     std::vector<GemmSet> m2m_c, m2m_c_t, l2l_c, l2l_c_t;  // per level
     // mixed: per-leaf L2P operators
     DBuf<float> E;
