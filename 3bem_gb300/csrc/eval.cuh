@@ -25,12 +25,18 @@
 namespace tbem {
 
 constexpr int EVAL_THREADS = 128;
+// threads per target: the whole CTA, or (template argument) given per item
+constexpr int EVAL_LONG = EVAL_THREADS, EVAL_PER_ITEM = 0;
 
 template <typename T>
 struct EvalArgs {
     // work items: CTA b handles task item_task[b], targets from item_start[b]
     const int* item_task;
     const int* item_start;
+    // EVAL_PER_ITEM launches: log2 of every item's threads per target, or
+    // (null) the one number for all
+    const int* item_tpt;
+    int tpt_log;
     // tasks
     const long* task_tgt;        // target block: first point, or cell id for surfaces
     const int* task_tgt_count;   // number of targets
@@ -146,7 +152,9 @@ __global__ void __launch_bounds__(EVAL_THREADS)
 eval_kernel(const EvalArgs<T> a)
 {
     constexpr int R = kernel_dim(KID);
-    constexpr int TPB = EVAL_THREADS / TPT;  // targets per CTA
+    // threads per target: a power of two, known at compile time or per item
+    const int tpt_log = TPT != EVAL_PER_ITEM ? 0 : a.item_tpt ? a.item_tpt[blockIdx.x] : a.tpt_log;
+    const int tpt = TPT != EVAL_PER_ITEM ? TPT : 1 << tpt_log;
     constexpr bool COMP = sizeof(T) == 4;    // compensated accumulation in FP32
     // scalar kernels with point sources and many right-hand sides: the
     // densities of four right-hand sides share one 4-vector, and the kernel
@@ -168,10 +176,10 @@ eval_kernel(const EvalArgs<T> a)
     const int task = a.item_task[blockIdx.x];
     const int t0 = a.item_start[blockIdx.x];
     const int ntgt = a.task_tgt_count[task];
-    const int lt = threadIdx.x / TPT;
-    const int lane = threadIdx.x % TPT;
+    const int lt = TPT != EVAL_PER_ITEM ? threadIdx.x / TPT : threadIdx.x >> tpt_log;
+    const int lane = TPT != EVAL_PER_ITEM ? threadIdx.x % TPT : threadIdx.x & (tpt - 1);
     const int ti = t0 + lt;
-    const bool active = lt < TPB && ti < ntgt;
+    const bool active = ti < ntgt;
     const double ox = a.task_origin[3 * task], oy = a.task_origin[3 * task + 1],
                  oz = a.task_origin[3 * task + 2];
     const long tb = a.task_tgt[task];
@@ -271,7 +279,7 @@ eval_kernel(const EvalArgs<T> a)
         __syncthreads();
         if (active) {
             const int n_here = min(EVAL_THREADS, total - tile);
-            for (int j = lane; j < n_here; j += TPT) {
+            for (int j = lane; j < n_here; j += tpt) {
                 const Vec4<T> q = sp[j];
                 if constexpr (DF) {
                     if (q.w != T(0)) {
@@ -341,7 +349,8 @@ eval_kernel(const EvalArgs<T> a)
     }
     // reduce the TPT partial sums of a target (consecutive lanes of one warp)
 #pragma unroll
-    for (int off = TPT / 2; off > 0; off /= 2) {
+    for (int off = 16; off > 0; off /= 2) {
+        if (off >= tpt) continue;
 #pragma unroll
         for (int i = 0; i < NR * R; i++) {
             T o = __shfl_xor_sync(0xffffffffu, acc[i], off);
@@ -353,6 +362,31 @@ eval_kernel(const EvalArgs<T> a)
             } else {
                 acc[i] += o;
             }
+        }
+    }
+    if (TPT == EVAL_PER_ITEM && tpt > 32) {
+        // one target per CTA: the warps' sums in warp order
+        constexpr int NW = EVAL_THREADS / 32;
+        __shared__ T red[2][NW][NR * R];
+        if (threadIdx.x % 32 == 0) {
+#pragma unroll
+            for (int i = 0; i < NR * R; i++) {
+                red[0][threadIdx.x / 32][i] = acc[i];
+                red[1][threadIdx.x / 32][i] = lo[i];
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < NW; w++)
+#pragma unroll
+                for (int i = 0; i < NR * R; i++) {
+                    if (COMP) {
+                        kahan_add(acc[i], lo[i], red[0][w][i]);
+                        lo[i] += red[1][w][i];
+                    } else {
+                        acc[i] += red[0][w][i];
+                    }
+                }
         }
     }
     if (!active || lane != 0) return;

@@ -11,8 +11,8 @@ struct EvalLaunch {
     bool tgt_surf;
     bool src_surf;
     int n_items;
-    int tpt = 4;  // threads per target (2, 4 or 8 for the point-to-point pass, 1, 2 or 4
-                  // for points to a check surface; 4 otherwise)
+    int tpt = 4;  // threads per target (point-to-point: EVAL_PER_ITEM in FP64, 2, 4 or 8 in FP32;
+                  // 1, 2 or 4 for points to a check surface; 4 otherwise)
 };
 
 // One function per kernel id (eval_k<id>.cu) so that the instantiations
@@ -42,14 +42,19 @@ constexpr int EVAL_NR_WIDE = 16;
 
 // Right-hand sides one launch of the evaluation kernel handles when
 // `remaining` are left from the launch's first one.
-inline int eval_rhs_block(int kid, bool fp32, bool trans, bool src_surf, int remaining)
+inline int eval_rhs_block(const EvalLaunch& L, bool fp32, int remaining)
 {
     if (remaining <= 1) return 1;
-    if (fp32 && kernel_dim(kid) == 1 && kernel_space_dim(kid) == 3 && !trans && !src_surf &&
+    if (fp32 && kernel_dim(L.kid) == 1 && kernel_space_dim(L.kid) == 3 && !L.trans && !L.src_surf &&
         remaining >= EVAL_NR_WIDE)
         return EVAL_NR_WIDE;
     return EVAL_NR;
 }
+
+// Threads per target of the direct sum: a warp until 32 targets per CTA give
+// every SM eight CTAs (with four threads per target, 6,144 points were 192 CTAs
+// on 152 SMs: traction 5.0 ms, 3.5 with a warp).
+inline int direct_tpt(long n_obs) { return n_obs < 152L * 8 * (EVAL_THREADS / 4) ? 32 : 4; }
 
 template <typename T>
 inline cudaError_t launch_eval(const EvalLaunch& L, const EvalArgs<T>& a, cudaStream_t s)

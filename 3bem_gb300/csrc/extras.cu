@@ -326,8 +326,9 @@ int tbem_direct_apply(int kernel, const double* kernel_params, const double* obs
             const int chunk = 1024;
             double org[3] = {0, 0, 0};
             for (long b = 0; b < n_obs; b += chunk)
-                ts.add(b, (int)std::min<long>(chunk, n_obs - b), org, {{0L, (int)n_src}}, EVAL_THREADS / 4);
-            ts.upload();
+                ts.add(b, (int)std::min<long>(chunk, n_obs - b), org, {{0L, (int)n_src}});
+            const int cut = TaskSet::SPLIT + direct_tpt(n_obs);
+            ts.upload({cut});
             EvalArgs<double> a{};
             ts.fill(a);
             a.t_xyz = ol.p;
@@ -342,7 +343,9 @@ int tbem_direct_apply(int kernel, const double* kernel_params, const double* obs
             a.add = 0;
             a.c2 = kp.c2;
             a.scale = kp.scale;
-            EvalLaunch L{kernel, false, false, false, ts.n_items()};
+            const TaskSet::Items& it = ts.cuts.at(cut);
+            TaskSet::fill_items(a, it);
+            EvalLaunch L{kernel, false, false, false, it.n, it.tpt};
             for (int r0 = 0; r0 < n_rhs; r0 += (n_rhs - r0 > 1 ? EVAL_NR : 1)) {
                 a.rhs0 = r0;
                 TBEM_CK(launch_eval<double>(L, a, s));

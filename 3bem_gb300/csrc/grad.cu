@@ -215,13 +215,14 @@ void with_kernel(int kid, F&& f)
 // (kernels with a source normal) in n_j are summed; the sums of c are
 // dL/dw_j.  The pass is paced by the FP64 pipe (two FMAs per SM and clock, 40
 // to 110 of them per pair), so what matters is that every SM has pairs: the
-// transposed task sets' work items (32 targets) are cut into GRAD_SUB CTAs of
-// one warp per target, whose lanes split its sources and meet in shuffles.  With one CTA of four threads per target per item and
+// task sets' work items are cut into CTAs of one warp per target, whose lanes
+// split its sources and meet in shuffles, or one target for the longest lists.  With one CTA of four threads per target per item and
 // forward-mode dual numbers through the kernel tensors, the four passes of
 // 6,144 sources and 4,096 observers took 28.4 ms in 107 to 182 CTAs; now 2.3 ms.
 struct GradEvalArgs {
     const int* item_task;
     const int* item_start;
+    const int* item_tpt;   // log2 of the item's threads per target
     const long* task_tgt;
     const int* task_tgt_count;
     const int* task_src_ptr;
@@ -250,9 +251,8 @@ struct GradEvalArgs {
     int obs_side;
     double* g;             // [t_n][7]: d/dposition (3), d/dnormal (3), value (1); accumulated
 };
-constexpr int GRAD_TPT = 32, GRAD_THREADS = 128;
-constexpr int GRAD_TARGETS = GRAD_THREADS / GRAD_TPT;           // targets per CTA
-constexpr int GRAD_SUB = (EVAL_THREADS / 4) / GRAD_TARGETS;     // CTAs per work item
+constexpr int GRAD_THREADS = 128, GRAD_WARPS = GRAD_THREADS / 32;
+static_assert(GRAD_THREADS == EVAL_LONG, "a long item is one target");
 
 template <int KID, bool OBS_SIDE, bool SRC_SURF>
 __global__ void __launch_bounds__(GRAD_THREADS) grad_eval_kernel(const GradEvalArgs a)
@@ -261,8 +261,9 @@ __global__ void __launch_bounds__(GRAD_THREADS) grad_eval_kernel(const GradEvalA
     constexpr int WN = OBS_SIDE ? (grad_obs_normal(KID) ? GN_OBS : GN_NONE) : (grad_src_normal(KID) ? GN_SRC : GN_NONE);
     constexpr bool NORMALS = normal_dot_kernel(KID);  // the kernel's value depends on a normal
     const int task = a.item_task[blockIdx.x];
-    const int ti = a.item_start[blockIdx.x] + (int)(blockIdx.y * GRAD_TARGETS + threadIdx.x / GRAD_TPT);
-    const int lane = threadIdx.x % GRAD_TPT;
+    const int tpt = 1 << a.item_tpt[blockIdx.x];  // 32 or GRAD_THREADS
+    const int ti = a.item_start[blockIdx.x] + (int)threadIdx.x / tpt;
+    const int lane = threadIdx.x % tpt;
     const bool active = ti < a.task_tgt_count[task];
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     if (active) {
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(GRAD_THREADS) grad_eval_kernel(const GradEvalA
 #pragma unroll
                 for (int k = 0; k < 3; k++) yc[k] = y[k] - a.s_center[3 * sb + k];
             }
-            for (int li = lane; li < cnt; li += GRAD_TPT) {
+            for (int li = lane; li < cnt; li += tpt) {
                 double dd[3], nz[3] = {0, 0, 0}, rv[3] = {0, 0, 0};
                 if (SRC_SURF) {
 #pragma unroll
@@ -329,9 +330,18 @@ __global__ void __launch_bounds__(GRAD_THREADS) grad_eval_kernel(const GradEvalA
         }
     }
 #pragma unroll
-    for (int off = GRAD_TPT / 2; off > 0; off /= 2)
+    for (int off = 16; off > 0; off /= 2)
 #pragma unroll
         for (int i = 0; i < 7; i++) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
+    if (tpt > 32) {  // one target per CTA: the warps' sums in warp order
+        __shared__ double red[GRAD_WARPS][7];
+        if (threadIdx.x % 32 == 0)
+            for (int i = 0; i < 7; i++) red[threadIdx.x / 32][i] = acc[i];
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < GRAD_WARPS; w++)
+                for (int i = 0; i < 7; i++) acc[i] += red[w][i];
+    }
     if (!active || lane != 0) return;
     double* g = a.g + 7 * (a.task_tgt[task] + ti);
 #pragma unroll
@@ -400,23 +410,24 @@ struct Out {
 // One transposed pass of the source gradients over a task set.
 void grad_pass(const TaskSet& ts, bool src_surf, GradEvalArgs a, cudaStream_t s, long* launches)
 {
-    if (ts.n_items() == 0) return;
-    a.item_task = ts.d_item_task.p;
-    a.item_start = ts.d_item_start.p;
-    a.task_tgt = ts.d_tgt.p;
-    a.task_tgt_count = ts.d_tgt_count.p;
-    a.task_src_ptr = ts.d_src_ptr.p;
-    a.src_blk = ts.d_blk.p;
-    a.src_blk_count = ts.d_blk_count.p;
-    const dim3 grid((unsigned)ts.n_items(), GRAD_SUB);
+    if (ts.empty()) return;
+    a.task_tgt = ts.d_tgt;
+    a.task_tgt_count = ts.d_tgt_count;
+    a.task_src_ptr = ts.d_src_ptr;
+    a.src_blk = ts.d_blk;
+    a.src_blk_count = ts.d_blk_count;
+    const TaskSet::Items& it = ts.cuts.at(TaskSet::SPLIT + 32);
+    a.item_task = it.task;
+    a.item_start = it.start;
+    a.item_tpt = it.tpt_log;
     with_kernel(a.kid, [&](auto K) {
         constexpr int kid = decltype(K)::value;
         if (a.obs_side) {
-            if (src_surf) grad_eval_kernel<kid, true, true><<<grid, GRAD_THREADS, 0, s>>>(a);
-            else grad_eval_kernel<kid, true, false><<<grid, GRAD_THREADS, 0, s>>>(a);
+            if (src_surf) grad_eval_kernel<kid, true, true><<<it.n, GRAD_THREADS, 0, s>>>(a);
+            else grad_eval_kernel<kid, true, false><<<it.n, GRAD_THREADS, 0, s>>>(a);
         } else {
-            if (src_surf) grad_eval_kernel<kid, false, true><<<grid, GRAD_THREADS, 0, s>>>(a);
-            else grad_eval_kernel<kid, false, false><<<grid, GRAD_THREADS, 0, s>>>(a);
+            if (src_surf) grad_eval_kernel<kid, false, true><<<it.n, GRAD_THREADS, 0, s>>>(a);
+            else grad_eval_kernel<kid, false, false><<<it.n, GRAD_THREADS, 0, s>>>(a);
         }
     });
     TBEM_CK(cudaGetLastError());

@@ -28,7 +28,6 @@ namespace {
 constexpr size_t NOALLOC_SCRATCH_BYTES = size_t(16) << 20;
 constexpr size_t NOALLOC_TASK_BYTES = size_t(1) << 20;     // work-item descriptors
 constexpr int NOALLOC_CHUNK = 1024;                        // observation points per task
-constexpr int NOALLOC_TPB = tbem::EVAL_THREADS / 4;        // targets per CTA (4 threads each)
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
 
@@ -71,7 +70,7 @@ TaskLayout layout(int n_tasks, int n_items)
 
 // One task per chunk of observation points, each against all sources.
 __global__ void noalloc_fill_tasks(unsigned char* base, TaskLayout L, long n_obs, int n_src,
-                                   int n_tasks, int n_items)
+                                   int n_tasks, int n_items, int tpb)
 {
     int* item_task = reinterpret_cast<int*>(base + L.item_task);
     int* item_start = reinterpret_cast<int*>(base + L.item_start);
@@ -82,11 +81,11 @@ __global__ void noalloc_fill_tasks(unsigned char* base, TaskLayout L, long n_obs
     long* blk = reinterpret_cast<long*>(base + L.blk);
     int* blk_count = reinterpret_cast<int*>(base + L.blk_count);
     int* blk_prefix = reinterpret_cast<int*>(base + L.blk_prefix);
-    const int per_task = NOALLOC_CHUNK / NOALLOC_TPB;
+    const int per_task = NOALLOC_CHUNK / tpb;  // tpb: targets per CTA
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n_items;
          i += (long)gridDim.x * blockDim.x) {
         item_task[i] = (int)(i / per_task);
-        item_start[i] = (int)(i % per_task) * NOALLOC_TPB;
+        item_start[i] = (int)(i % per_task) * tpb;
     }
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t <= n_tasks;
          t += (long)gridDim.x * blockDim.x) {
@@ -146,8 +145,8 @@ extern "C" int tbem_direct_apply_noalloc(int kernel, const double* kernel_params
                                           " doubles");
         const long n_tasks = (n_obs + NOALLOC_CHUNK - 1) / NOALLOC_CHUNK;
         const long last = n_obs - (n_tasks - 1) * NOALLOC_CHUNK;
-        const long n_items = (n_tasks - 1) * (NOALLOC_CHUNK / NOALLOC_TPB) +
-                             (last + NOALLOC_TPB - 1) / NOALLOC_TPB;
+        const int tpt = direct_tpt(n_obs), tpb = EVAL_THREADS / tpt;
+        const long n_items = (n_tasks - 1) * (NOALLOC_CHUNK / tpb) + (last + tpb - 1) / tpb;
         const TaskLayout TL = layout((int)std::min<long>(n_tasks, INT32_MAX),
                                      (int)std::min<long>(n_items, INT32_MAX));
         if (n_items > INT32_MAX || TL.total > NOALLOC_TASK_BYTES)
@@ -165,7 +164,7 @@ extern "C" int tbem_direct_apply_noalloc(int kernel, const double* kernel_params
         cudaStream_t s = (cudaStream_t)stream;
 
         noalloc_fill_tasks<<<(unsigned)std::min<long>((n_items + 255) / 256 + 1, 4096), 256, 0, s>>>(
-            base, TL, n_obs, (int)n_src, (int)n_tasks, (int)n_items);
+            base, TL, n_obs, (int)n_src, (int)n_tasks, (int)n_items, tpb);
         TBEM_CK(cudaGetLastError());
         const long total = (long)R * n_src * n_rhs;
         if (total > 0) {
@@ -179,6 +178,8 @@ extern "C" int tbem_direct_apply_noalloc(int kernel, const double* kernel_params
         EvalArgs<double> a{};
         a.item_task = reinterpret_cast<const int*>(base + TL.item_task);
         a.item_start = reinterpret_cast<const int*>(base + TL.item_start);
+        a.item_tpt = nullptr;
+        a.tpt_log = tpt == 32 ? 5 : 2;
         a.task_tgt = reinterpret_cast<const long*>(base + TL.task_tgt);
         a.task_tgt_count = reinterpret_cast<const int*>(base + TL.task_count);
         a.task_origin = reinterpret_cast<const double*>(base + TL.task_origin);
@@ -198,7 +199,7 @@ extern "C" int tbem_direct_apply_noalloc(int kernel, const double* kernel_params
         a.add = 0;
         a.c2 = kp.c2;
         a.scale = kp.scale;
-        EvalLaunch L{kernel, false, false, false, (int)n_items};
+        EvalLaunch L{kernel, false, false, false, (int)n_items, EVAL_PER_ITEM};
         for (int r0 = 0; r0 < n_rhs; r0 += (n_rhs - r0 > 1 ? EVAL_NR : 1)) {
             a.rhs0 = r0;
             TBEM_CK(launch_eval<double>(L, a, s));

@@ -49,13 +49,11 @@ void check_cusolver(cusolverStatus_t e, const char* what, const char* file, int 
 // ------------------------------------------------------------------ helpers
 
 void TaskSet::add(long target, int count, const double* org,
-                  const std::vector<std::pair<long, int>>& srcs, int targets_per_cta,
-                  const std::vector<int>& near)
+                  const std::vector<std::pair<long, int>>& srcs, const std::vector<int>& near)
 {
     int pre = 0;
     for (auto& s : srcs) pre += std::max(s.second, 0);
     if (count <= 0 || pre == 0) return;
-    const int t = (int)tgt.size();
     tgt.push_back(target);
     tgt_count.push_back(count);
     origin.insert(origin.end(), org, org + 3);
@@ -74,27 +72,93 @@ void TaskSet::add(long target, int count, const double* org,
     }
     src_ptr.push_back((int)blk.size());
     n_pairs += (long)count * pre;
-    for (int st = 0; st < count; st += targets_per_cta) {
-        item_task.push_back(t);
-        item_start.push_back(st);
-    }
 }
 
-void TaskSet::upload()
+// A CTA walks its task's sources in total / tpt steps, whatever its number of
+// targets, so a pass lasts at least as long as its longest list.  On the
+// bumpy sphere of 61,440 points two coarse leaves see 60,965 sources against
+// 1,592 at the median: the SMs idled for 47 % of the FP64 near field behind
+// their CTAs.  A task whose steps exceed an even share of the set's steps
+// over EVAL_SLOTS resident CTAs (and EVAL_MIN_STEPS, about what starting a
+// CTA costs) therefore runs with a warp per target, or, where even that
+// exceeds it, the whole CTA per target (gradient passes of 6,144 sources and
+// 4,096 observers: 4.64 ms for the whole gradient without, 4.09 with).
+namespace {
+constexpr long EVAL_SLOTS = 152 * 8, EVAL_MIN_STEPS = 32;
+}
+
+void TaskSet::upload(const std::vector<int>& tpts)
 {
-    d_tgt.upload(tgt);
-    d_tgt_count.upload(tgt_count);
-    d_origin.upload(origin);
-    d_src_ptr.upload(src_ptr);
-    d_blk.upload(blk);
-    d_blk_count.upload(blk_count);
-    d_blk_prefix.upload(blk_prefix);
-    if (!blk_near.empty()) {
-        blk_near.resize(blk.size(), 0);
-        d_blk_near.upload(blk_near);
+    const int nt = n_tasks();
+    std::vector<int> total(nt);
+    for (int t = 0; t < nt; t++) {
+        const int last = src_ptr[t + 1] - 1;
+        total[t] = blk_prefix[last] + blk_count[last];
     }
-    d_item_task.upload(item_task);
-    d_item_start.upload(item_start);
+    table = PackedTable();
+    struct Pending {
+        int key, tpt, n;
+        size_t task, start, log;
+    };
+    std::vector<Pending> pending;
+    for (int key : tpts) {
+        const bool split = key >= SPLIT;
+        const int base = split ? key - SPLIT : key;
+        std::vector<int> task, start, log;
+        auto cut_task = [&](int t, int tpt) {
+            int lg = 0;
+            while ((1 << lg) < tpt) lg++;
+            for (int st = 0; st < tgt_count[t]; st += EVAL_THREADS / tpt) {
+                task.push_back(t);
+                start.push_back(st);
+                if (split) log.push_back(lg);
+            }
+        };
+        if (!split) {
+            for (int t = 0; t < nt; t++) cut_task(t, base);
+        } else {
+            long steps = 0;  // of the whole set with `base` threads per target
+            for (int t = 0; t < nt; t++)
+                steps += (long)((tgt_count[t] * base + EVAL_THREADS - 1) / EVAL_THREADS) * ((total[t] + base - 1) / base);
+            const long cap = std::max(EVAL_MIN_STEPS, steps / EVAL_SLOTS);
+            std::vector<std::pair<int, int>> order(nt);  // (steps, task), longest first
+            std::vector<int> tpt(nt);
+            for (int t = 0; t < nt; t++) {
+                tpt[t] = total[t] <= cap * base ? base : total[t] <= cap * 32 ? std::max(base, 32) : EVAL_LONG;
+                order[t] = {total[t] / tpt[t], t};
+            }
+            std::stable_sort(order.begin(), order.end(),
+                             [](const auto& a, const auto& b) { return a.first > b.first; });
+            for (const auto& o : order) cut_task(o.second, tpt[o.second]);
+        }
+        if (!task.empty()) {
+            const size_t ot = table.add(task), os = table.add(start), ol = table.add(log);
+            pending.push_back({key, split ? EVAL_PER_ITEM : base, (int)task.size(), ot, os, ol});
+        }
+    }
+    const size_t o_tgt = table.add(tgt), o_cnt = table.add(tgt_count), o_org = table.add(origin),
+                 o_ptr = table.add(src_ptr), o_blk = table.add(blk), o_bc = table.add(blk_count),
+                 o_bp = table.add(blk_prefix);
+    if (!blk_near.empty()) blk_near.resize(blk.size(), 0);
+    const size_t o_near = table.add(blk_near);
+    table.upload();
+    d_tgt = table.at<long>(o_tgt);
+    d_tgt_count = table.at<int>(o_cnt);
+    d_origin = table.at<double>(o_org);
+    d_src_ptr = table.at<int>(o_ptr);
+    d_blk = table.at<long>(o_blk);
+    d_blk_count = table.at<int>(o_bc);
+    d_blk_prefix = table.at<int>(o_bp);
+    d_blk_near = blk_near.empty() ? nullptr : table.at<int>(o_near);
+    cuts.clear();
+    for (const Pending& q : pending) {
+        Items& it = cuts[q.key];
+        it.tpt = q.tpt;
+        it.n = q.n;
+        it.task = table.at<int>(q.task);
+        it.start = table.at<int>(q.start);
+        it.tpt_log = q.tpt == EVAL_PER_ITEM ? table.at<int>(q.log) : nullptr;
+    }
 }
 
 void GemmSet::add_group(long a_off, const std::vector<std::pair<int, int>>& pairs)
@@ -694,7 +758,7 @@ Plan::~Plan()
     if (solver) cusolverDnDestroy(solver);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
-    if (side) cudaStreamDestroy(side);
+    if (aux) cudaStreamDestroy(aux);
     if (stream) cudaStreamDestroy(stream);
     if (own) cudaSetDevice(prev);
 }
@@ -830,7 +894,10 @@ void Plan::build(int kernel, const double* params, const double* obs_locs,
 void Plan::create_streams()
 {
     TBEM_CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    TBEM_CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    int least = 0, greatest = 0;
+    TBEM_CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    TBEM_CK(cudaStreamCreateWithPriority(&aux, cudaStreamNonBlocking,
+                                         opt.precision == TBEM_PRECISION_FP64 ? greatest : least));
     TBEM_CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
     TBEM_CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
     TBEM_CKB(cublasCreate(&cublas));
@@ -1021,12 +1088,11 @@ void Plan::autotune_tc()
 }
 
 namespace {
-// A timed variant replaces the best one so far only when it is clearly faster:
-// near ties (variants within about 1 % on a 100 us pass, where repeated
-// timings differ by as much) would otherwise fall either way from one
-// construction to the next, and with them the summation order, which the plain
-// form's pseudo-inverses turn into 1e-8 of the result.
-constexpr float AUTOTUNE_MARGIN = 0.97f;
+// A timed variant replaces the best one so far only when it is faster by more
+// than repeated timings differ: variants that tie would otherwise fall either
+// way from one construction to the next, and with them the summation order,
+// which the plain form's pseudo-inverses turn into 1e-8 of the result.
+constexpr float AUTOTUNE_MARGIN = 0.995f;
 }  // namespace
 
 // Picks the point-to-point pass's threads per target (2, 4 or 8) by timing
@@ -1034,7 +1100,7 @@ constexpr float AUTOTUNE_MARGIN = 0.97f;
 // does not depend on the values).
 void Plan::autotune_p2p()
 {
-    if (p2p.n_items() == 0) return;
+    if (p2p.empty()) return;
     ensure_rhs(1);
     const bool mixed = f.mixed && !f.f64;  // FP32 evaluation passes
     if (mixed) TBEM_CK(cudaMemsetAsync(s32.p, 0, sizeof(float) * R * n_src, stream));
@@ -1046,14 +1112,14 @@ void Plan::autotune_p2p()
     for (int tpt : {4, 2, 8}) {
         p2p_tpt = tpt;
         float ms = 1e30f;
-        for (int rep = 0; rep < 4; rep++) {
+        for (int rep = 0; rep < 5; rep++) {
             TBEM_CK(cudaEventRecord(e0, stream));
             if (mixed)
-                eval<float>(p2p_set(), kid, false, false, otree, dobs, 0, *dsrc, 0, s32.p, n_src,
-                            nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false);
+                eval<float>(p2p, kid, false, false, otree, dobs, 0, *dsrc, 0, s32.p, n_src,
+                            nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, p2p_tpt);
             else
-                eval<double>(p2p_set(), kid, false, false, otree, dobs, 0, *dsrc, 0, s64.p, n_src,
-                             nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false);
+                eval<double>(p2p, kid, false, false, otree, dobs, 0, *dsrc, 0, s64.p, n_src,
+                             nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, p2p_tpt);
             TBEM_CK(cudaEventRecord(e1, stream));
             TBEM_CK(cudaEventSynchronize(e1));
             float t = 0.f;
@@ -1072,7 +1138,7 @@ void Plan::autotune_p2p()
 // the same way: each variant timed on this operator's own leaves.
 void Plan::autotune_p2m()
 {
-    if (p2m.n_items() == 0) return;
+    if (p2m.empty()) return;
     ensure_rhs(1);
     const bool mixed = f.mixed && !f.f64;  // FP32 evaluation passes
     if (mixed) TBEM_CK(cudaMemsetAsync(s32.p, 0, sizeof(float) * R * n_src, stream));
@@ -1084,14 +1150,14 @@ void Plan::autotune_p2m()
     for (int tpt : {4, 2, 1}) {
         p2m_tpt = tpt;
         float ms = 1e30f;
-        for (int rep = 0; rep < 4; rep++) {
+        for (int rep = 0; rep < 5; rep++) {
             TBEM_CK(cudaEventRecord(e0, stream));
             if (mixed)
-                eval<float>(p2m_set(), f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s32.p, n_src,
-                            nullptr, nullptr, 0, cu32.p, 0, 1, stream, false);
+                eval<float>(p2m, f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s32.p, n_src,
+                            nullptr, nullptr, 0, cu32.p, 0, 1, stream, false, p2m_tpt);
             else
-                eval<double>(p2m_set(), f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s64.p, n_src,
-                             nullptr, nullptr, 0, cu64.p, 0, 1, stream, false);
+                eval<double>(p2m, f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s64.p, n_src,
+                             nullptr, nullptr, 0, cu64.p, 0, 1, stream, false, p2m_tpt);
             TBEM_CK(cudaEventRecord(e1, stream));
             TBEM_CK(cudaEventSynchronize(e1));
             float t = 0.f;
@@ -1110,13 +1176,10 @@ void Plan::build_tasks()
 {
     const Tree& O = otree;
     const Tree& S = *stree;
-    constexpr int TPB = EVAL_THREADS / 4;
     // forward
     for (int c : L.p2m) {
         const Cell& cc = S.cells[c];
-        p2m.add(c, ns, cc.center, {{cc.pt_begin, (int)cc.n_points()}}, TPB);
-        p2m_tpt1.add(c, ns, cc.center, {{cc.pt_begin, (int)cc.n_points()}}, EVAL_THREADS);
-        p2m_tpt2.add(c, ns, cc.center, {{cc.pt_begin, (int)cc.n_points()}}, EVAL_THREADS / 2);
+        p2m.add(c, ns, cc.center, {{cc.pt_begin, (int)cc.n_points()}});
     }
     std::vector<std::vector<int>> p2p_of(O.cells.size()), m2p_of(O.cells.size()),
         p2l_of(O.cells.size()), m2l_of(O.cells.size());
@@ -1229,27 +1292,25 @@ void Plan::build_tasks()
             }
             for (int s : m2p_of[a]) mp.push_back({s, ns});
         }
-        p2p.add(leaf.pt_begin, (int)leaf.n_points(), leaf.center, pp, TPB, near);
-        p2p_tpt2.add(leaf.pt_begin, (int)leaf.n_points(), leaf.center, pp, EVAL_THREADS / 2, near);
-        p2p_tpt8.add(leaf.pt_begin, (int)leaf.n_points(), leaf.center, pp, EVAL_THREADS / 8, near);
-        m2p.add(leaf.pt_begin, (int)leaf.n_points(), leaf.center, mp, TPB);
+        p2p.add(leaf.pt_begin, (int)leaf.n_points(), leaf.center, pp, near);
+        m2p.add(leaf.pt_begin, (int)leaf.n_points(), leaf.center, mp);
     }
     for (size_t c = 0; c < O.cells.size(); c++) {
         const Cell& oc = O.cells[c];
         std::vector<std::pair<long, int>> pl, ml;
         for (int s : p2l_of[c]) pl.push_back({S.cells[s].pt_begin, (int)S.cells[s].n_points()});
         for (int s : m2l_of[c]) ml.push_back({s, ns});
-        p2l.add((long)c, ns, oc.center, pl, TPB);
-        if (f.m2l_on_the_fly) m2l_fly.add((long)c, ns, oc.center, ml, TPB);
+        p2l.add((long)c, ns, oc.center, pl);
+        if (f.m2l_on_the_fly) m2l_fly.add((long)c, ns, oc.center, ml);
     }
     for (int c : L.l2p) {
         const Cell& cc = O.cells[c];
-        l2p.add(cc.pt_begin, (int)cc.n_points(), cc.center, {{c, ns}}, TPB);
+        l2p.add(cc.pt_begin, (int)cc.n_points(), cc.center, {{c, ns}});
     }
     // transposed: targets live in the source tree, sources in the observation tree
     for (int c : L.p2m) {
         const Cell& cc = S.cells[c];
-        p2m_t.add(cc.pt_begin, (int)cc.n_points(), cc.center, {{c, ns}}, TPB);
+        p2m_t.add(cc.pt_begin, (int)cc.n_points(), cc.center, {{c, ns}});
     }
     for (size_t c = 0; c < S.cells.size(); c++) {
         const Cell& leaf = S.cells[c];
@@ -1259,28 +1320,36 @@ void Plan::build_tasks()
             for (int o : p2p_by_src[a]) pp.push_back({O.cells[o].pt_begin, (int)O.cells[o].n_points()});
             for (int o : p2l_by_src[a]) pl.push_back({o, ns});
         }
-        p2p_t.add(leaf.pt_begin, (int)leaf.n_points(), leaf.center, pp, TPB);
-        p2l_t.add(leaf.pt_begin, (int)leaf.n_points(), leaf.center, pl, TPB);
+        p2p_t.add(leaf.pt_begin, (int)leaf.n_points(), leaf.center, pp);
+        p2l_t.add(leaf.pt_begin, (int)leaf.n_points(), leaf.center, pl);
     }
     for (size_t c = 0; c < S.cells.size(); c++) {
         const Cell& sc = S.cells[c];
         std::vector<std::pair<long, int>> mp, ml;
         for (int o : m2p_by_src[c]) mp.push_back({O.cells[o].pt_begin, (int)O.cells[o].n_points()});
         for (int o : m2l_by_src[c]) ml.push_back({o, ns});
-        m2p_t.add((long)c, ns, sc.center, mp, TPB);
-        if (f.m2l_on_the_fly) m2l_fly_t.add((long)c, ns, sc.center, ml, TPB);
+        m2p_t.add((long)c, ns, sc.center, mp);
+        if (f.m2l_on_the_fly) m2l_fly_t.add((long)c, ns, sc.center, ml);
     }
     for (int c : L.l2p) {
         const Cell& cc = O.cells[c];
-        l2p_t.add(c, ns, cc.center, {{cc.pt_begin, (int)cc.n_points()}}, TPB);
+        l2p_t.add(c, ns, cc.center, {{cc.pt_begin, (int)cc.n_points()}});
     }
-    p2p_tpt2.tpt = 2;
-    p2p_tpt8.tpt = 8;
-    p2m_tpt1.tpt = 1;
-    p2m_tpt2.tpt = 2;
-    for (TaskSet* t : {&p2m, &p2m_tpt1, &p2m_tpt2, &p2p, &p2p_tpt2, &p2p_tpt8, &m2p, &p2l, &l2p, &m2l_fly, &p2m_t, &p2p_t,
-                       &m2p_t, &p2l_t, &l2p_t, &m2l_fly_t})
-        t->upload();
+    // the near field's long lists are split in FP64 (the FP64 forms' applies,
+    // every form's gradient passes); the FP32 passes keep one cut, whose
+    // order of summation their results show at 1e-7
+    // (the gradient passes: a warp per target at least)
+    constexpr int SP = TaskSet::SPLIT;
+    if (opt.precision == TBEM_PRECISION_MIXED) {
+        p2p.upload({2, 4, 8, SP + 32});
+        p2p_t.upload({4, SP + 32});
+    } else {
+        p2p.upload({SP + 2, SP + 4, SP + 8, SP + 32});
+        p2p_t.upload({SP + 4, SP + 32});
+    }
+    p2m.upload({1, 2, 4});
+    for (TaskSet* t : {&m2p, &l2p, &p2m_t, &p2l_t}) t->upload({4, SP + 32});
+    for (TaskSet* t : {&p2l, &m2l_fly, &m2p_t, &l2p_t, &m2l_fly_t}) t->upload({4});
 
     // dedup keys of the M2M / L2L octant translations and the M2L translations
     const int LS = S.n_levels(), LO = O.n_levels();
@@ -2571,9 +2640,9 @@ template <typename T>
 void Plan::eval(const TaskSet& ts, int ekid, bool tgt_surf, bool src_surf, const Tree&,
                 const DTree& dt, double t_rref, const DTree& ds, double s_rref, const T* s_str,
                 long s_n, const T* q, double* y, long y_n, T* c, int add, int nrhs,
-                cudaStream_t s, bool trans)
+                cudaStream_t s, bool trans, int tpt)
 {
-    if (ts.n_items() == 0) return;
+    if (ts.empty()) return;
     EvalArgs<T> a{};
     ts.fill(a);
     a.t_xyz = dt.xyz.p;
@@ -2600,12 +2669,17 @@ void Plan::eval(const TaskSet& ts, int ekid, bool tgt_surf, bool src_surf, const
     const KParams ep = make_kparams(ekid, mu, nu);
     a.c2 = T(ep.c2);
     a.scale = ep.scale;
-    EvalLaunch Lc{ekid, trans, tgt_surf, src_surf, ts.n_items()};
-    Lc.tpt = ts.tpt;
-    for (int r0 = 0; r0 < nrhs; r0 += eval_rhs_block(ekid, sizeof(T) == 4, trans, src_surf, nrhs - r0)) {
+    // the FP64 passes take the cut with the long lists split where there is one
+    auto cut = sizeof(T) == 8 ? ts.cuts.find(TaskSet::SPLIT + tpt) : ts.cuts.end();
+    if (cut == ts.cuts.end()) cut = ts.cuts.find(tpt);
+    const TaskSet::Items& it = cut->second;
+    TaskSet::fill_items(a, it);
+    EvalLaunch Lc{ekid, trans, tgt_surf, src_surf, it.n, it.tpt};
+    for (int r0 = 0; r0 < nrhs;) {
         a.rhs0 = r0;
         TBEM_CK(launch_eval<T>(Lc, a, s));
         launches++;
+        r0 += eval_rhs_block(Lc, sizeof(T) == 4, nrhs - r0);
     }
 }
 
@@ -2628,35 +2702,35 @@ void Plan::forward(int nrhs, cudaStream_t s)
         TBEM_CK(cudaMemsetAsync(cu64.p, 0, sizeof(double) * ncs * nrhs * n, s));
         TBEM_CK(cudaMemsetAsync(cd64.p, 0, sizeof(double) * nco * nrhs * n, s));
         mark("gather", s);
-        // the near field on the side stream: it fills the SMs that the upward
-        // pass, a chain of small launches, leaves idle
+        // the far field on the second stream, the near field on this one
+        const cudaStream_t far = aux;
         TBEM_CK(cudaEventRecord(ev_fork, s));
-        TBEM_CK(cudaStreamWaitEvent(side, ev_fork, 0));
-        eval<double>(p2p_set(), kid, false, false, O, dobs, 0, *dsrc, 0, s64.p, NS, nullptr, y64.p, NO, nullptr, 1, nrhs, side, false);
-        TBEM_CK(cudaEventRecord(ev_join, side));
-        eval<double>(p2m_set(), F.ks_kid, true, false, S, *dsrc, F.r_uc, *dsrc, 0, s64.p, NS, nullptr, nullptr, 0, cu64.p, 0, nrhs, s, false);
-        mark("p2m", s);
+        TBEM_CK(cudaStreamWaitEvent(aux, ev_fork, 0));
+        eval<double>(p2m, F.ks_kid, true, false, S, *dsrc, F.r_uc, *dsrc, 0, s64.p, NS, nullptr, nullptr, 0, cu64.p, 0, nrhs, far, false, p2m_tpt);
+        mark("p2m", far);
+        eval<double>(p2p, kid, false, false, O, dobs, 0, *dsrc, 0, s64.p, NS, nullptr, y64.p, NO, nullptr, 1, nrhs, s, false, p2p_tpt);
         for (int l = S.n_levels() - 1; l >= 0; l--) {
-            if (l < (int)F.m2m.size()) F.m2m_slots[l].run(qu64.p, cu64.p, n, nrhs, 0, slots64.p, s, &launches);
-            F.c2e_up[l].run<double>(cu64.p, qu64.p, n, nrhs, 0, GEMM_STORE, s, &launches);
+            if (l < (int)F.m2m.size()) F.m2m_slots[l].run(qu64.p, cu64.p, n, nrhs, 0, slots64.p, far, &launches);
+            F.c2e_up[l].run<double>(cu64.p, qu64.p, n, nrhs, 0, GEMM_STORE, far, &launches);
         }
-        mark("m2m+c2e_up", s);
-        // join the near field: the passes below add into the same outputs
-        TBEM_CK(cudaStreamWaitEvent(s, ev_join, 0));
-        mark("p2p", s);
-        eval<double>(m2p, F.kt_kid, false, true, O, dobs, 0, *dsrc, F.r_ue, nullptr, 0, qu64.p, y64.p, NO, nullptr, 1, nrhs, s, false);
-        eval<double>(p2l, F.ks_kid, true, false, O, dobs, F.r_dc, *dsrc, 0, s64.p, NS, nullptr, nullptr, 0, cd64.p, 1, nrhs, s, false);
-        mark("m2p+p2l", s);
+        mark("m2m+c2e_up", far);
+        eval<double>(p2l, F.ks_kid, true, false, O, dobs, F.r_dc, *dsrc, 0, s64.p, NS, nullptr, nullptr, 0, cd64.p, 1, nrhs, far, false);
+        mark("p2l", far);
         if (F.m2l_on_the_fly)
-            eval<double>(m2l_fly, F.g_kid, true, true, O, dobs, F.r_dc, *dsrc, F.r_ue, nullptr, 0, qu64.p, nullptr, 0, cd64.p, 1, nrhs, s, false);
+            eval<double>(m2l_fly, F.g_kid, true, true, O, dobs, F.r_dc, *dsrc, F.r_ue, nullptr, 0, qu64.p, nullptr, 0, cd64.p, 1, nrhs, far, false);
         else
-            F.m2l_slots.run(qu64.p, cd64.p, n, nrhs, 0, slots64.p, s, &launches);
-        mark("m2l", s);
+            F.m2l_slots.run(qu64.p, cd64.p, n, nrhs, 0, slots64.p, far, &launches);
+        mark("m2l", far);
         for (int l = 0; l < O.n_levels(); l++) {
-            if (l > 0 && l - 1 < (int)F.l2l.size()) F.l2l[l - 1].run<double>(qd64.p, cd64.p, n, nrhs, 0, GEMM_ADD, s, &launches);
-            F.c2e_dn[l].run<double>(cd64.p, qd64.p, n, nrhs, 0, GEMM_STORE, s, &launches);
+            if (l > 0 && l - 1 < (int)F.l2l.size()) F.l2l[l - 1].run<double>(qd64.p, cd64.p, n, nrhs, 0, GEMM_ADD, far, &launches);
+            F.c2e_dn[l].run<double>(cd64.p, qd64.p, n, nrhs, 0, GEMM_STORE, far, &launches);
         }
-        mark("l2l+c2e_down", s);
+        mark("l2l+c2e_down", far);
+        // join: the passes below read the far field and add into the near field's outputs
+        TBEM_CK(cudaEventRecord(ev_join, aux));
+        TBEM_CK(cudaStreamWaitEvent(s, ev_join, 0));
+        mark("p2p_wait", s);
+        eval<double>(m2p, F.kt_kid, false, true, O, dobs, 0, *dsrc, F.r_ue, nullptr, 0, qu64.p, y64.p, NO, nullptr, 1, nrhs, s, false);
         eval<double>(l2p, F.kt_kid, false, true, O, dobs, 0, dobs, F.r_de, nullptr, 0, qd64.p, y64.p, NO, nullptr, 1, nrhs, s, false);
         mark("l2p", s);
     } else {
@@ -2666,7 +2740,7 @@ void Plan::forward(int nrhs, cudaStream_t s)
         TBEM_CK(cudaMemsetAsync(cu32.p, 0, sizeof(float) * ncs * nrhs * n, s));
         TBEM_CK(cudaMemsetAsync(cd32.p, 0, sizeof(float) * nco * nrhs * n, s));
         mark("gather", s);
-        eval<float>(p2m_set(), F.ks_kid, true, false, S, *dsrc, F.r_uc, *dsrc, 0, s32.p, NS, nullptr, nullptr, 0, cu32.p, 0, nrhs, s, false);
+        eval<float>(p2m, F.ks_kid, true, false, S, *dsrc, F.r_uc, *dsrc, 0, s32.p, NS, nullptr, nullptr, 0, cu32.p, 0, nrhs, s, false, p2m_tpt);
         mark("p2m", s);
         for (int l = S.n_levels() - 1; l >= 0; l--) {
             if (l >= (int)F.m2m.size() || F.m2m[l].empty()) continue;
@@ -2682,7 +2756,7 @@ void Plan::forward(int nrhs, cudaStream_t s)
             }
         }
         mark("m2m", s);
-        eval<float>(p2p_set(), kid, false, false, O, dobs, 0, *dsrc, 0, s32.p, NS, nullptr, y64.p, NO, nullptr, 1, nrhs, s, false);
+        eval<float>(p2p, kid, false, false, O, dobs, 0, *dsrc, 0, s32.p, NS, nullptr, y64.p, NO, nullptr, 1, nrhs, s, false, p2p_tpt);
         mark("p2p", s);
         const bool need64 = !L.m2p.empty() || F.m2l_on_the_fly;
         if (need64) {
@@ -2752,31 +2826,32 @@ void Plan::adjoint(int nrhs, cudaStream_t s)
         launches++;
         TBEM_CK(cudaMemsetAsync(qu64.p, 0, sizeof(double) * ncs * nrhs * n, s));
         TBEM_CK(cudaMemsetAsync(qd64.p, 0, sizeof(double) * nco * nrhs * n, s));
-        // L2P^T, M2P^T, P2P^T
-        eval<double>(l2p_t, F.kt_kid, true, false, O, dobs, F.r_de, dobs, 0, y64.p, NO, nullptr, nullptr, 0, qd64.p, 1, nrhs, s, true);
-        eval<double>(m2p_t, F.kt_kid, true, false, S, *dsrc, F.r_ue, dobs, 0, y64.p, NO, nullptr, nullptr, 0, qu64.p, 1, nrhs, s, true);
-        // the near field on the side stream, joined before the passes that add
-        // into the same outputs
+        // the far field on the second stream, the near field on this one
+        const cudaStream_t far = aux;
         TBEM_CK(cudaEventRecord(ev_fork, s));
-        TBEM_CK(cudaStreamWaitEvent(side, ev_fork, 0));
-        eval<double>(p2p_t, kid, false, false, S, *dsrc, 0, dobs, 0, y64.p, NO, nullptr, s64.p, NS, nullptr, 1, nrhs, side, true);
-        TBEM_CK(cudaEventRecord(ev_join, side));
+        TBEM_CK(cudaStreamWaitEvent(aux, ev_fork, 0));
+        // L2P^T, M2P^T, P2P^T
+        eval<double>(l2p_t, F.kt_kid, true, false, O, dobs, F.r_de, dobs, 0, y64.p, NO, nullptr, nullptr, 0, qd64.p, 1, nrhs, far, true);
+        eval<double>(m2p_t, F.kt_kid, true, false, S, *dsrc, F.r_ue, dobs, 0, y64.p, NO, nullptr, nullptr, 0, qu64.p, 1, nrhs, far, true);
+        eval<double>(p2p_t, kid, false, false, S, *dsrc, 0, dobs, 0, y64.p, NO, nullptr, s64.p, NS, nullptr, 1, nrhs, s, true);
         // down pass reversed: deepest level first
         for (int l = O.n_levels() - 1; l >= 0; l--) {
-            F.c2e_dn_t[l].run<double>(qd64.p, cd64.p, n, nrhs, 1, GEMM_STORE, s, &launches);
-            if (l > 0 && l - 1 < (int)F.l2l_t.size()) F.l2l_t_slots[l - 1].run(cd64.p, qd64.p, n, nrhs, 1, slots64.p, s, &launches);
+            F.c2e_dn_t[l].run<double>(qd64.p, cd64.p, n, nrhs, 1, GEMM_STORE, far, &launches);
+            if (l > 0 && l - 1 < (int)F.l2l_t.size()) F.l2l_t_slots[l - 1].run(cd64.p, qd64.p, n, nrhs, 1, slots64.p, far, &launches);
         }
         if (F.m2l_on_the_fly)
-            eval<double>(m2l_fly_t, F.g_kid, true, true, S, *dsrc, F.r_ue, dobs, F.r_dc, nullptr, 0, cd64.p, nullptr, 0, qu64.p, 1, nrhs, s, true);
+            eval<double>(m2l_fly_t, F.g_kid, true, true, S, *dsrc, F.r_ue, dobs, F.r_dc, nullptr, 0, cd64.p, nullptr, 0, qu64.p, 1, nrhs, far, true);
         else
-            F.m2l_t_slots.run(cd64.p, qu64.p, n, nrhs, 1, slots64.p, s, &launches);
-        TBEM_CK(cudaStreamWaitEvent(s, ev_join, 0));
-        eval<double>(p2l_t, F.ks_kid, false, true, S, *dsrc, 0, dobs, F.r_dc, nullptr, 0, cd64.p, s64.p, NS, nullptr, 1, nrhs, s, true);
+            F.m2l_t_slots.run(cd64.p, qu64.p, n, nrhs, 1, slots64.p, far, &launches);
         // up pass reversed: root first
         for (int l = 0; l < S.n_levels(); l++) {
-            F.c2e_up_t[l].run<double>(qu64.p, cu64.p, n, nrhs, 1, GEMM_STORE, s, &launches);
-            if (l < (int)F.m2m_t.size()) F.m2m_t[l].run<double>(cu64.p, qu64.p, n, nrhs, 1, GEMM_ADD, s, &launches);
+            F.c2e_up_t[l].run<double>(qu64.p, cu64.p, n, nrhs, 1, GEMM_STORE, far, &launches);
+            if (l < (int)F.m2m_t.size()) F.m2m_t[l].run<double>(cu64.p, qu64.p, n, nrhs, 1, GEMM_ADD, far, &launches);
         }
+        // join: the passes below add into the near field's outputs
+        TBEM_CK(cudaEventRecord(ev_join, aux));
+        TBEM_CK(cudaStreamWaitEvent(s, ev_join, 0));
+        eval<double>(p2l_t, F.ks_kid, false, true, S, *dsrc, 0, dobs, F.r_dc, nullptr, 0, cd64.p, s64.p, NS, nullptr, 1, nrhs, s, true);
         eval<double>(p2m_t, F.ks_kid, false, true, S, *dsrc, 0, *dsrc, F.r_uc, nullptr, 0, cu64.p, s64.p, NS, nullptr, 1, nrhs, s, true);
     } else {
         gather_kernel<float><<<grid_for(NO * R * nrhs), 256, 0, s>>>(xin, dobs.perm.p, nullptr, s32.p, NO, R, nrhs);
@@ -2858,40 +2933,41 @@ void Plan::forward_compressed(int nrhs, cudaStream_t s)
     TBEM_CK(cudaMemsetAsync(cuc, 0, sizeof(T) * ncs * nrhs * ri, s));
     TBEM_CK(cudaMemsetAsync(cdc, 0, sizeof(T) * nco * nrhs * ro, s));
     mark("gather", s);
-    // the near field on the side stream, beside the far-field passes below
+    // the near field on the second stream, the far field on this one
+    const cudaStream_t far = s, near = aux;
     TBEM_CK(cudaEventRecord(ev_fork, s));
-    TBEM_CK(cudaStreamWaitEvent(side, ev_fork, 0));
-    eval<T>(p2p_set(), kid, false, false, O, dobs, 0, *dsrc, 0, str, NS, nullptr, y64.p, NO, nullptr, 1, nrhs, side, false);
-    TBEM_CK(cudaEventRecord(ev_join, side));
+    TBEM_CK(cudaStreamWaitEvent(aux, ev_fork, 0));
+    eval<T>(p2p, kid, false, false, O, dobs, 0, *dsrc, 0, str, NS, nullptr, y64.p, NO, nullptr, 1, nrhs, near, false, p2p_tpt);
     // P2M into the leaves' check potentials, then u~ = P_l u
-    eval<T>(p2m_set(), F.ks_kid, true, false, S, *dsrc, F.r_uc, *dsrc, 0, str, NS, nullptr, nullptr, 0, cu, 0, nrhs, s, false);
-    F.comp_p2m.run_rect<T>(cu, cuc, ri, n, n, nrhs, 0, GEMM_ATOMIC, s, &launches);  // into zeros
-    mark("p2m", s);
+    eval<T>(p2m, F.ks_kid, true, false, S, *dsrc, F.r_uc, *dsrc, 0, str, NS, nullptr, nullptr, 0, cu, 0, nrhs, far, false, p2m_tpt);
+    F.comp_p2m.run_rect<T>(cu, cuc, ri, n, n, nrhs, 0, GEMM_ATOMIC, far, &launches);  // into zeros
+    mark("p2m", far);
     for (int l = S.n_levels() - 1; l >= 0; l--)
-        if (l < (int)F.m2m_c.size()) F.m2m_c[l].run_rect<T>(cuc, cuc, ri, ri, ri, nrhs, 0, GEMM_ATOMIC, s, &launches);
-    mark("m2m", s);
+        if (l < (int)F.m2m_c.size()) F.m2m_c[l].run_rect<T>(cuc, cuc, ri, ri, ri, nrhs, 0, GEMM_ATOMIC, far, &launches);
+    mark("m2m", far);
     if (!L.p2l.empty()) {
-        TBEM_CK(cudaMemsetAsync(cd, 0, sizeof(T) * nco * nrhs * n, s));
-        eval<T>(p2l, F.ks_kid, true, false, O, dobs, F.r_dc, *dsrc, 0, str, NS, nullptr, nullptr, 0, cd, 1, nrhs, s, false);
-        F.comp_p2l.run_rect<T>(cd, cdc, ro, n, ro, nrhs, 1, GEMM_ATOMIC, s, &launches);
+        TBEM_CK(cudaMemsetAsync(cd, 0, sizeof(T) * nco * nrhs * n, far));
+        eval<T>(p2l, F.ks_kid, true, false, O, dobs, F.r_dc, *dsrc, 0, str, NS, nullptr, nullptr, 0, cd, 1, nrhs, far, false);
+        F.comp_p2l.run_rect<T>(cd, cdc, ro, n, ro, nrhs, 1, GEMM_ATOMIC, far, &launches);
     }
-    mark("m2p+p2l", s);
+    mark("m2p+p2l", far);
     bool tc_done = false;
     if constexpr (sizeof(T) == 4) {
         if (F.use_tc_c) {
-            F.tc_c.split_b_rows(cuc, 0, ncs * nrhs, std::max(ncs, nco) * nrhs, s);
+            F.tc_c.split_b_rows(cuc, 0, ncs * nrhs, std::max(ncs, nco) * nrhs, far);
             launches++;
-            mark("m2l_split", s);
-            F.m2l_c.run_tc(F.tc_c, cdc, nrhs, 1, (long)ro * ri, s, &launches);
+            mark("m2l_split", far);
+            F.m2l_c.run_tc(F.tc_c, cdc, nrhs, 1, (long)ro * ri, far, &launches);
             tc_done = true;
         }
     }
-    if (!tc_done) F.m2l_c.run_rect<T>(cuc, cdc, ro, ri, ri, nrhs, 0, GEMM_ATOMIC, s, &launches);
-    mark("m2l", s);
+    if (!tc_done) F.m2l_c.run_rect<T>(cuc, cdc, ro, ri, ri, nrhs, 0, GEMM_ATOMIC, far, &launches);
+    mark("m2l", far);
     for (int l = 1; l < O.n_levels(); l++)
-        if (l - 1 < (int)F.l2l_c.size()) F.l2l_c[l - 1].run_rect<T>(cdc, cdc, ro, ro, ro, nrhs, 0, GEMM_ATOMIC, s, &launches);
-    mark("l2l", s);
-    // join the near field: the passes below add into the same outputs
+        if (l - 1 < (int)F.l2l_c.size()) F.l2l_c[l - 1].run_rect<T>(cdc, cdc, ro, ro, ro, nrhs, 0, GEMM_ATOMIC, far, &launches);
+    mark("l2l", far);
+    // join: the passes below read the far field and add into the near field's outputs
+    TBEM_CK(cudaEventRecord(ev_join, aux));
     TBEM_CK(cudaStreamWaitEvent(s, ev_join, 0));
     mark("p2p_wait", s);
     if (!L.m2p.empty()) {
@@ -2933,65 +3009,62 @@ void Plan::adjoint_compressed(int nrhs, cudaStream_t s)
     launches++;
     TBEM_CK(cudaMemsetAsync(cuc, 0, sizeof(T) * ncs * nrhs * ri, s));
     TBEM_CK(cudaMemsetAsync(cdc, 0, sizeof(T) * nco * nrhs * ro, s));
-    // the near field on the side stream, as in the forward apply
+    // the near field on the second stream, the far field on this one
+    const cudaStream_t far = s, near = aux;
     TBEM_CK(cudaEventRecord(ev_fork, s));
-    TBEM_CK(cudaStreamWaitEvent(side, ev_fork, 0));
-    eval<T>(p2p_t, kid, false, false, S, *dsrc, 0, dobs, 0, zin, NO, nullptr, s64.p, NS, nullptr, 1, nrhs, side, true);
-    TBEM_CK(cudaEventRecord(ev_join, side));
-    bool joined = false;
-    auto join = [&] {  // before the passes that add into the same outputs
-        if (!joined) TBEM_CK(cudaStreamWaitEvent(s, ev_join, 0));
-        joined = true;
-    };
+    TBEM_CK(cudaStreamWaitEvent(aux, ev_fork, 0));
     if (F.n_l2p > 0) {
-        launch_l2p_t(zin, ro, nrhs, cdc, s);
+        launch_l2p_t(zin, ro, nrhs, cdc, far);
     }
+    eval<T>(p2p_t, kid, false, false, S, *dsrc, 0, dobs, 0, zin, NO, nullptr, s64.p, NS, nullptr, 1, nrhs, near, true);
     for (int l = O.n_levels() - 1; l >= 1; l--)
-        if (l - 1 < (int)F.l2l_c_t.size()) F.l2l_c_t[l - 1].run_rect<T>(cdc, cdc, ro, ro, ro, nrhs, 1, GEMM_ATOMIC, s, &launches);
+        if (l - 1 < (int)F.l2l_c_t.size()) F.l2l_c_t[l - 1].run_rect<T>(cdc, cdc, ro, ro, ro, nrhs, 1, GEMM_ATOMIC, far, &launches);
     // C_k^T on the tensor cores from the forward planes, as the forward M2L
     bool tc_done = false;
     if constexpr (sizeof(T) == 4) {
         if (F.use_tc_c) {
-            F.tc_c.split_b_rows(cdc, 0, nco * nrhs, std::max(ncs, nco) * nrhs, s, true);
+            F.tc_c.split_b_rows(cdc, 0, nco * nrhs, std::max(ncs, nco) * nrhs, far, true);
             launches++;
-            F.m2l_c_t.run_tc(F.tc_c, cuc, nrhs, 1, (long)ro * ri, s, &launches, true);
+            F.m2l_c_t.run_tc(F.tc_c, cuc, nrhs, 1, (long)ro * ri, far, &launches, true);
             tc_done = true;
         }
     }
-    if (!tc_done) F.m2l_c_t.run_rect<T>(cdc, cuc, ri, ro, ri, nrhs, 1, GEMM_ATOMIC, s, &launches);
+    if (!tc_done) F.m2l_c_t.run_rect<T>(cdc, cuc, ri, ro, ri, nrhs, 1, GEMM_ATOMIC, far, &launches);
     if (!L.p2l.empty()) {
-        F.comp_p2l.run_rect<T>(cdc, cd, n, ro, ro, nrhs, 0, GEMM_STORE, s, &launches);
-        join();
-        eval<T>(p2l_t, F.ks_kid, false, true, S, *dsrc, 0, dobs, F.r_dc, nullptr, 0, cd, s64.p, NS, nullptr, 1, nrhs, s, true);
+        F.comp_p2l.run_rect<T>(cdc, cd, n, ro, ro, nrhs, 0, GEMM_STORE, far, &launches);
     }
     if (!L.m2p.empty()) {
         // density gradients in FP64, folded into u~ through (2^-l W)^T
-        TBEM_CK(cudaMemsetAsync(qu64.p, 0, sizeof(double) * ncs * nrhs * n, s));
+        TBEM_CK(cudaMemsetAsync(qu64.p, 0, sizeof(double) * ncs * nrhs * n, far));
         if constexpr (sizeof(T) == 4) {
-            gather_kernel<double><<<grid_for(NO * R * nrhs), 256, 0, s>>>(xin, dobs.perm.p, nullptr, y64.p, NO, R, nrhs);
+            gather_kernel<double><<<grid_for(NO * R * nrhs), 256, 0, far>>>(xin, dobs.perm.p, nullptr, y64.p, NO, R, nrhs);
             TBEM_CK(cudaGetLastError());
             launches++;
         }
-        eval<double>(m2p_t, F.kt_kid, true, false, S, *dsrc, F.r_ue, dobs, 0, y64.p, NO, nullptr, nullptr, 0, qu64.p, 1, nrhs, s, true);
+        eval<double>(m2p_t, F.kt_kid, true, false, S, *dsrc, F.r_ue, dobs, 0, y64.p, NO, nullptr, nullptr, 0, qu64.p, 1, nrhs, far, true);
         if constexpr (sizeof(T) == 4) {
-            TBEM_CK(cudaMemsetAsync(cu, 0, sizeof(float) * ncs * nrhs * n, s));
-            add_kernel<<<grid_for(ncs * nrhs * n), 256, 0, s>>>(qu64.p, cu, ncs * nrhs * n);
+            TBEM_CK(cudaMemsetAsync(cu, 0, sizeof(float) * ncs * nrhs * n, far));
+            add_kernel<<<grid_for(ncs * nrhs * n), 256, 0, far>>>(qu64.p, cu, ncs * nrhs * n);
             TBEM_CK(cudaGetLastError());
             launches++;
-            F.decomp_m2p.run_rect<float>(cu, cuc, ri, n, ri, nrhs, 1, GEMM_ATOMIC, s, &launches);
+            F.decomp_m2p.run_rect<float>(cu, cuc, ri, n, ri, nrhs, 1, GEMM_ATOMIC, far, &launches);
         } else {
-            F.decomp_m2p.run_rect<double>(qu64.p, cuc, ri, n, ri, nrhs, 1, GEMM_ATOMIC, s, &launches);
+            F.decomp_m2p.run_rect<double>(qu64.p, cuc, ri, n, ri, nrhs, 1, GEMM_ATOMIC, far, &launches);
         }
     }
     for (int l = 0; l < S.n_levels(); l++)
-        if (l < (int)F.m2m_c_t.size()) F.m2m_c_t[l].run_rect<T>(cuc, cuc, ri, ri, ri, nrhs, 1, GEMM_ATOMIC, s, &launches);
+        if (l < (int)F.m2m_c_t.size()) F.m2m_c_t[l].run_rect<T>(cuc, cuc, ri, ri, ri, nrhs, 1, GEMM_ATOMIC, far, &launches);
     // the compression set skips the P2M leaves whose states reach no result
     // (their transposed states are zero), but the transposed P2M below reads
     // every P2M leaf: clear the buffer first (it still holds the M2P densities
     // or an earlier apply's values)
-    TBEM_CK(cudaMemsetAsync(cu, 0, sizeof(T) * ncs * nrhs * n, s));
-    F.comp_p2m.run_rect<T>(cuc, cu, n, ri, n, nrhs, 1, GEMM_STORE, s, &launches);
-    join();
+    TBEM_CK(cudaMemsetAsync(cu, 0, sizeof(T) * ncs * nrhs * n, far));
+    F.comp_p2m.run_rect<T>(cuc, cu, n, ri, n, nrhs, 1, GEMM_STORE, far, &launches);
+    // join: the passes below add into the near field's outputs
+    TBEM_CK(cudaEventRecord(ev_join, aux));
+    TBEM_CK(cudaStreamWaitEvent(s, ev_join, 0));
+    if (!L.p2l.empty())
+        eval<T>(p2l_t, F.ks_kid, false, true, S, *dsrc, 0, dobs, F.r_dc, nullptr, 0, cd, s64.p, NS, nullptr, 1, nrhs, s, true);
     eval<T>(p2m_t, F.ks_kid, false, true, S, *dsrc, 0, *dsrc, F.r_uc, nullptr, 0, cu, s64.p, NS, nullptr, 1, nrhs, s, true);
 }
 
@@ -3112,7 +3185,7 @@ void Plan::sync(cudaStream_t s)
     DeviceGuard guard(opt.device);
     if (s) TBEM_CK(cudaStreamSynchronize(s));
     TBEM_CK(cudaStreamSynchronize(stream));
-    TBEM_CK(cudaStreamSynchronize(side));
+    TBEM_CK(cudaStreamSynchronize(aux));
     const std::vector<const int*> flags = device_flags();
     bool raised = flags_raised();
     for (size_t i = 0; i < flags.size(); i++) {

@@ -177,7 +177,8 @@ struct ScopedEvent {
     }
 };
 
-// A set of obs-owner evaluation tasks (eval.cuh).
+// A set of obs-owner evaluation tasks (eval.cuh) and the work items (CTAs) it
+// is cut into for each number of threads per target it may run with.
 struct TaskSet {
     std::vector<long> tgt;
     std::vector<int> tgt_count;
@@ -186,32 +187,53 @@ struct TaskSet {
     std::vector<long> blk;
     std::vector<int> blk_count, blk_prefix;
     std::vector<int> blk_near;  // per block: its cell touches the target leaf (point-to-point sets)
-    std::vector<int> item_task, item_start;
-    DBuf<long> d_tgt, d_blk;
-    DBuf<int> d_tgt_count, d_src_ptr, d_blk_count, d_blk_prefix, d_item_task, d_item_start, d_blk_near;
-    DBuf<double> d_origin;
+    PackedTable table;
+    const long *d_tgt = nullptr, *d_blk = nullptr;
+    const int *d_tgt_count = nullptr, *d_src_ptr = nullptr, *d_blk_count = nullptr, *d_blk_prefix = nullptr,
+              *d_blk_near = nullptr;
+    const double* d_origin = nullptr;
     long n_pairs = 0;  // sum over tasks of targets x sources (work estimate)
-    int tpt = 4;       // threads per target the items were cut for
+
+    // One launch: n CTAs, CTA b handles EVAL_THREADS / tpt targets of task
+    // task[b] from its target start[b] on, tpt the same for all of them or
+    // (EVAL_PER_ITEM) 2^tpt_log[b].
+    struct Items {
+        int tpt = 4, n = 0;
+        const int *task = nullptr, *start = nullptr, *tpt_log = nullptr;
+    };
+    // per number of threads per target its launch; + SPLIT: per item, more
+    // threads for the tasks of long source lists
+    static constexpr int SPLIT = 1024;
+    std::map<int, Items> cuts;
 
     int n_tasks() const { return (int)tgt.size(); }
-    int n_items() const { return (int)item_task.size(); }
+    bool empty() const { return tgt.empty(); }
     // near: one flag per entry of srcs (empty: no flags)
     void add(long target, int count, const double* org, const std::vector<std::pair<long, int>>& srcs,
-             int targets_per_cta, const std::vector<int>& near = {});
-    void upload();
+             const std::vector<int>& near = {});
+    // Cuts the tasks for each number of threads per target in `tpts` and
+    // copies everything in.  + SPLIT: tasks whose source lists are long
+    // against an even share of the chip get a warp or a CTA (EVAL_LONG) per
+    // target instead, and the items run longest first.
+    void upload(const std::vector<int>& tpts);
     template <typename T>
     void fill(EvalArgs<T>& a) const
     {
-        a.item_task = d_item_task.p;
-        a.item_start = d_item_start.p;
-        a.task_tgt = d_tgt.p;
-        a.task_tgt_count = d_tgt_count.p;
-        a.task_origin = d_origin.p;
-        a.task_src_ptr = d_src_ptr.p;
-        a.src_blk = d_blk.p;
-        a.src_blk_count = d_blk_count.p;
-        a.src_blk_prefix = d_blk_prefix.p;
-        a.src_blk_near = d_blk_near.p;
+        a.task_tgt = d_tgt;
+        a.task_tgt_count = d_tgt_count;
+        a.task_origin = d_origin;
+        a.task_src_ptr = d_src_ptr;
+        a.src_blk = d_blk;
+        a.src_blk_count = d_blk_count;
+        a.src_blk_prefix = d_blk_prefix;
+        a.src_blk_near = d_blk_near;
+    }
+    template <typename T>
+    static void fill_items(EvalArgs<T>& a, const Items& it)
+    {
+        a.item_task = it.task;
+        a.item_start = it.start;
+        a.item_tpt = it.tpt_log;
     }
 };
 
@@ -388,17 +410,11 @@ struct Plan {
     Form f;
     // evaluation task sets (forward); adjoint sets swap roles
     TaskSet p2m, p2p, m2p, p2l, l2p, m2l_fly;
-    // point-to-point variants for 2 and 8 threads per target (autotuned)
-    TaskSet p2p_tpt2, p2p_tpt8;
-    int p2p_tpt = 4;
-    // points-to-check-surface variants for 1 and 2 threads per target (autotuned)
-    TaskSet p2m_tpt1, p2m_tpt2;
-    int p2m_tpt = 4;
+    int p2p_tpt = 4;  // threads per target of the point-to-point pass (2, 4 or 8; autotuned)
+    int p2m_tpt = 4;  // and of the points-to-check-surface pass (1, 2 or 4)
     void autotune_p2m();
-    const TaskSet& p2m_set() const { return p2m_tpt == 1 ? p2m_tpt1 : p2m_tpt == 2 ? p2m_tpt2 : p2m; }
     void autotune_p2p();
     void autotune_tc();  // N tile (128 / 64) of the tensor-core translations
-    const TaskSet& p2p_set() const { return p2p_tpt == 2 ? p2p_tpt2 : p2p_tpt == 8 ? p2p_tpt8 : p2p; }
     TaskSet p2m_t, p2p_t, m2p_t, p2l_t, l2p_t, m2l_fly_t;
     // work buffers
     int cap_rhs = 0;
@@ -414,10 +430,15 @@ struct Plan {
     DBuf<float> cuc32, cdc32;  // compressed M2L coefficients [cell][rhs][r_in | r_out]
     DBuf<double> cuc64, cdc64;  // the same in the FP64 compressed form
     cudaStream_t stream = nullptr;
-    // second stream for the near field, which runs beside the far-field
-    // passes of the compressed form (forked after the gather, joined before
-    // the passes that add into the outputs)
-    cudaStream_t side = nullptr;
+    // Near and far field run side by side on the apply's stream and this one
+    // (forked after the gather, joined before the passes that add into the
+    // outputs).  The compressed forms put the near field here: the far field
+    // is their longer chain and keeps the apply's stream without the two event
+    // hops.  The plain form puts the far field here, with the device's highest
+    // priority: its chains of small launches would queue behind the thousands
+    // of CTAs of the near field (15,360-point sphere: 8.1 ms without, 7.7 with;
+    // a batch of 16 meshes in the precision form: 12.9 and 13.4).
+    cudaStream_t aux = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cublasHandle_t cublas = nullptr;
     cusolverDnHandle_t solver = nullptr;
@@ -519,7 +540,7 @@ struct Plan {
     void eval(const TaskSet& ts, int ekid, bool tgt_surf, bool src_surf, const Tree& tt,
               const DTree& dt, double t_rref, const DTree& ds, double s_rref, const T* s_str,
               long s_n, const T* q, double* y, long y_n, T* c, int add, int nrhs, cudaStream_t s,
-              bool trans);
+              bool trans, int tpt = 4);
     void mark(const char* name, cudaStream_t s);
     template <typename T>
     void launch_l2p(const T* cd, int len, int nrhs, cudaStream_t s);
