@@ -352,6 +352,7 @@ int tbem_fmm_set_wait_cycles(TbemFmm* h, long long cycles)
     if (cycles < 0) return fail(TBEM_ERR_ARG, "negative wait budget");
     h->plan.f.tc.wait_cycles = cycles;
     h->plan.f.tc_c.wait_cycles = cycles;
+    h->plan.f.oz.wait_cycles = cycles;
     return TBEM_OK;
 }
 

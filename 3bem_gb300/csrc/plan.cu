@@ -1988,6 +1988,15 @@ void Plan::build_mixed_ops(Form& F)
         F.tc_c.build(F.Cops.p, n_m2l_ops, F.r_out, F.r_in, stream);
         TBEM_CK(cudaStreamSynchronize(stream));
     }
+    // the FP64 compressed form's M2L from digit planes on the tensor cores
+    // while they (16 bytes per value, twice the operators') stay within 64 GB;
+    // m2l_path 4 keeps the FP64 pipe
+    F.use_oz = F.f64 && opt.m2l_path != 4 && n_m2l_ops > 0 &&
+               16.0 * n_m2l_ops * ((F.r_out + 127) / 128 * 128) * ((F.r_in + 31) / 32 * 32) <= 64e9;
+    if (F.use_oz) {
+        F.oz.build(F.Cops64.p, n_m2l_ops, F.r_out, F.r_in, stream);
+        TBEM_CK(cudaStreamSynchronize(stream));
+    }
     // the auto path keeps the M2L products on the tensor cores when they do
     // not compress (uncompressed 3xBF16 planes)
     const bool auto_tc = opt.m2l_path == 0 && !F.f64 && !F.m2l_compressed && !F.m2l_on_the_fly &&
@@ -2960,6 +2969,12 @@ void Plan::forward_compressed(int nrhs, cudaStream_t s)
             F.m2l_c.run_tc(F.tc_c, cdc, nrhs, 1, (long)ro * ri, far, &launches);
             tc_done = true;
         }
+    } else if (F.use_oz) {
+        F.oz.split_b(cuc, ncs * nrhs, far);
+        launches++;
+        mark("m2l_split", far);
+        F.m2l_c.run_oz(F.oz, cdc, nrhs, far, &launches);
+        tc_done = true;
     }
     if (!tc_done) F.m2l_c.run_rect<T>(cuc, cdc, ro, ri, ri, nrhs, 0, GEMM_ATOMIC, far, &launches);
     mark("m2l", far);
@@ -3124,6 +3139,7 @@ int Plan::rhs_chunk(int nrhs) const
     double per = 8.0 * R * N * 4;  // io copies, strengths, outputs
     if (f.f64) {
         per += 8.0 * (ncs * n + ncs * f.r_in + nco * f.r_out);
+        if (f.use_oz) per += 16.0 * ncs * f.oz.k_pad;
         if (!L.p2l.empty()) per += 8.0 * nco * n;
         if (!L.m2p.empty()) per += 8.0 * ncs * n;
     } else if (f.mixed) {
@@ -3168,6 +3184,7 @@ std::vector<const int*> Plan::device_flags() const
     std::vector<const int*> v;
     if (f.tc.err.p) v.push_back(f.tc.err.p);
     if (f.tc_c.err.p) v.push_back(f.tc_c.err.p);
+    if (f.oz.err.p) v.push_back(f.oz.err.p);
     return v;
 }
 

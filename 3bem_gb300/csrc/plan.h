@@ -252,6 +252,20 @@ struct TcPlanes {
                       bool trans = false);
 };
 
+// Digit planes of the FP64 compressed form's M2L operators for the tensor-core
+// FP64 GEMM (oz_gemm.cu), plus the digits of the current B operand.
+struct OzPlanes {
+    static constexpr int S = 8;  // digits per value
+    int m = 0, k = 0, m_pad = 0, k_pad = 0;
+    long n_ops = 0, b_digit = 0;
+    DBuf<__nv_bfloat16> a, b;
+    DBuf<int> a_exp, b_exp;
+    DBuf<int> err;              // set by a GEMM whose bounded wait gave up
+    long long wait_cycles = 0;  // budget of its bounded waits (0: the default)
+    void build(const double* ops, long n_ops, int m, int k, cudaStream_t s);
+    void split_b(const double* cells, long rows, cudaStream_t s);
+};
+
 // A set of GEMM groups (gemm.cuh) sharing B and D buffers.
 struct GemmSet {
     std::vector<long> A_off;  // operator offsets (elements) into an operator pool
@@ -291,6 +305,9 @@ struct GemmSet {
     // trans: op(A) = A^T (B from planes split with trans, D columns of P.k rows)
     void run_tc(const TcPlanes& P, float* D, int nrhs, int atomic, long nn, cudaStream_t s,
                 long* launches, bool trans = false);
+    // FP64 products through the digit planes, added atomically into D
+    std::map<int, DBuf<int4>> oz_tiles;  // per nrhs
+    void run_oz(const OzPlanes& P, double* D, int nrhs, cudaStream_t s, long* launches);
 };
 
 // Deterministic accumulation of a GEMM set whose groups add into the same
@@ -373,6 +390,8 @@ struct Form {
     // operators kept in FP64 and applied on the FP64 pipes
     bool f64 = false;
     DBuf<double> Pb64, Wl64, Vb64, Cops64, Xops64, Yops64, E64;
+    OzPlanes oz;  // digit planes of Cops64 (use_oz: the M2L runs through them)
+    bool use_oz = false;
     DBuf<double> V64;  // V in FP64 (column-major n x r_out) while the L2P operators are built
     GemmSet m2l_c, m2l_c_t, comp_p2m, decomp_m2p, comp_p2l;
     GemmSet decomp_l2p;  // V over the L2P leaves: their down-check potentials (gradients)
