@@ -166,6 +166,12 @@ eval_kernel(const EvalArgs<T> a)
     // the double layer's pairs with a source block touching the target leaf:
     // double-float n . d (lapd_near_df), the block's flag in the position's w
     constexpr bool DF = SPLIT && KID == LAP_D && !TRANS;
+    // point-to-point in FP64 for a traction kernel: three multiply-adds per
+    // component; n.v of a source rides in its density's w where the kernel
+    // takes the source normal
+    constexpr bool TRAC64 = !COMP && !SRC_SURF && !TGT_SURF &&
+                            (KID == EL_TRAC || KID == EL_ADJ || KID == EL_TRAC2 || KID == EL_ADJ2);
+    constexpr bool SRC_N = (KID == EL_TRAC || KID == EL_TRAC2) != TRANS;  // the kernel's normal is the source's
     // per source: position, normal, and the R density components of every
     // right-hand side, each a 4-vector (one shared load in the pair loop)
     __shared__ Vec4<T> sp[EVAL_THREADS], sn[EVAL_THREADS];
@@ -258,7 +264,8 @@ eval_kernel(const EvalArgs<T> a)
 #pragma unroll
                         for (int d = 0; d < R; d++)
                             vv[d] = r_ < nr_here ? a.s_str[((long)(a.rhs0 + r_) * R + d) * a.s_n + p] : T(0);
-                        sv[r_][threadIdx.x] = Vec4<T>{vv[0], vv[1], vv[2], T(0)};
+                        const T nv = TRAC64 && SRC_N ? nx * vv[0] + ny * vv[1] + nz * vv[2] : T(0);
+                        sv[r_][threadIdx.x] = Vec4<T>{vv[0], vv[1], vv[2], nv};
                     }
                 }
             }
@@ -328,7 +335,16 @@ eval_kernel(const EvalArgs<T> a)
                     // transposed apply: the target is the forward source and
                     // the source the forward observer, so the separation
                     // (forward src - forward obs) flips sign and the normals swap
-                    if (TRANS)
+                    if constexpr (TRAC64) {
+                        const T sg = TRANS ? T(-1) : T(1);
+                        if constexpr (SRC_N)
+                            accumulate_traction<KID, TRANS, T>(sg * dx, sg * dy, sg * dz, nq.x, nq.y, nq.z, vq.w,
+                                                               a.c2, v, &part[r_ * R]);
+                        else
+                            accumulate_traction<KID, TRANS, T>(sg * dx, sg * dy, sg * dz, pnx, pny, pnz,
+                                                               pnx * v[0] + pny * v[1] + pnz * v[2], a.c2, v,
+                                                               &part[r_ * R]);
+                    } else if (TRANS)
                         accumulate<KID, true, T>(-dx, -dy, -dz, nq.x, nq.y, nq.z, pnx, pny, pnz,
                                                  a.c2, v, &part[r_ * R]);
                     else

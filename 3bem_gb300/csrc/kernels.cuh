@@ -268,6 +268,32 @@ __device__ __forceinline__ void accumulate(T dx, T dy, T dz, T nox, T noy, T noz
     }
 }
 
+// The traction kernels as three multiply-adds per component, for the passes
+// that the FP64 pipe paces (two FMAs per SM and clock): with s = -1 (traction,
+// m = n_y) or +1 (adjoint traction, m = n_x) and t = c2 / r^q (q = 3, in 2D 2),
+//   K v = s t (m.d) v + (s q (m.d)(d.v) / r^(q+2) + t m.v) d - t (d.v) m,
+// the signs of the last two t terms flipped for K^T.  accumulate() evaluates
+// the same products component by component, with 21 operations where this has
+// 9 in 3D.  mv = m.v.
+template <int KID, bool TRANS, typename T>
+__device__ __forceinline__ void accumulate_traction(T dx, T dy, T dz, T mx, T my, T mz, T mv, T c2, const T* v, T* u)
+{
+    constexpr bool D3 = kernel_space_dim(KID) == 3;
+    constexpr bool TRAC = KID == EL_TRAC || KID == EL_TRAC2;
+    const T r2 = D3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
+    if (r2 < T(1e-12)) return;
+    const T ir = dev_rsqrt<T>(r2);
+    const T ir2 = ir * ir, irq = D3 ? ir2 * ir : ir2;
+    const T dm = D3 ? dx * mx + dy * my + dz * mz : dx * mx + dy * my;
+    const T dv = D3 ? dx * v[0] + dy * v[1] + dz * v[2] : dx * v[0] + dy * v[1];
+    const T t = c2 * irq, w = (TRAC ? -irq : irq) * dm;
+    const T al = c2 * w, ga = TRANS ? t * dv : -t * dv;
+    const T be = (T(D3 ? 3 : 2) * ir2 * dv) * w + (TRANS ? -t * mv : t * mv);
+    u[0] += al * v[0] + be * dx + ga * mx;
+    u[1] += al * v[1] + be * dy + ga * my;
+    if (D3) u[2] += al * v[2] + be * dz + ga * mz;
+}
+
 // Full tensor (row-major R x C, constant included) for operator assembly.
 template <typename T>
 __device__ __forceinline__ void kernel_tensor(int kid, T dx, T dy, T dz, T nox, T noy, T noz,
