@@ -13,7 +13,8 @@
 //
 // FP32 (grouped_gemm_kernel): CTA of 256 threads, tile BM x 64 (BM = 128 or
 // 64: the choice that pads m the least), each thread an (BM / 16) x 4 block of
-// outputs.  FP64: dgemm_warp_kernel below, tiles of one warp.  A launch with too
+// outputs; launches of few tiles: small_gemm_kernel.  FP64: dgemm_warp_kernel,
+// tiles of one warp.  A launch with too
 // few tiles to fill the GPU splits K over blockIdx.z (partial products added
 // atomically).  K runs in steps of
 // BK through two shared-memory buffers: the next step's global loads are in
@@ -209,6 +210,138 @@ inline int gemm_bm(int m)
 {
     const int p128 = (m + 127) / 128 * 128, p64 = (m + 63) / 64 * 64;
     return p64 < p128 ? 64 : 128;
+}
+
+// ------------------------------------------------- FP32 GEMM, few columns
+//
+// The level sums of one operator and one right-hand side are small products
+// (64 to 4,096 columns of 256 rows), paced by latency: with 64-wide tiles a
+// launch is 8 to 128 CTAs, each waiting for L2 once per 16 depths.  Tiles of 32 x 32 by
+// 64 threads (4 x 4 outputs each, rows tm + 8 i and columns tn + 8 j) spread
+// the launch over the chip, and three stages of 32 depths filled by cp.async
+// keep two steps in flight (eight CTAs per SM).  Both tiles stay depth-contiguous as they
+// lie in memory, rows padded to 36 floats: the 16-byte reads of a warp touch
+// every bank once.  A thread multiplies 4 rows x 4 columns x 4
+// depths between eight shared loads; every output is one chain over ascending
+// depth, over the same split of the depth as the large tiles' (run_rect), so
+// both sum alike.  B columns are read in 16-byte pieces (a depth of a multiple
+// of four), A too (VA) unless it is transposed.  98,304-point fault, per
+// operator: the M2M levels 38 + 18 + 15 + 12 us with the large tiles, 22 + 11 +
+// 8 + 7 now; a 960-point sphere's compression (56 columns) 14.5 and 7.1.
+constexpr int SG_B = 32, SG_K = 32, SG_PAD = SG_K + 4, SG_STAGES = 3, SG_THREADS = 64;
+
+__device__ __forceinline__ void sg_copy16(float* dst, const float* src, bool in)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(in ? 16u : 0u)
+                 : "memory");
+}
+__device__ __forceinline__ void sg_copy4(float* dst, const float* src, bool in)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(in ? 4u : 0u)
+                 : "memory");
+}
+
+template <bool VA>
+__global__ void __launch_bounds__(SG_THREADS) small_gemm_kernel(const GemmArgs<float> a)
+{
+    __shared__ __align__(16) float As[SG_STAGES][SG_B][SG_PAD], Bs[SG_STAGES][SG_B][SG_PAD];
+    const int tid = threadIdx.x, tm = tid % 8, tn = tid / 8;
+    const int g = a.tile_group[blockIdx.x], col0 = a.tile_col0[blockIdx.x];
+    const int m0 = blockIdx.y * SG_B, M = a.m, K = a.k, lda = a.lda;
+    const float* __restrict__ A = a.A[g];
+    const long pair0 = a.g_pair0[g];
+    const int ncols = a.g_npairs[g] * a.nrhs;
+    const int kb = blockIdx.z * a.kchunk, kend = min(K, kb + a.kchunk);
+    const int steps = (kend - kb + SG_K - 1) / SG_K;
+
+    const float* bcol[4];  // this thread's B columns: tid / 8 + 8 i of the tile
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int c = col0 + tid / 8 + 8 * i;
+        bcol[i] = nullptr;
+        if (c < ncols) {
+            const int p = c / a.nrhs, r = c - p * a.nrhs;
+            bcol[i] = a.B + ((long)a.in_cell[pair0 + p] * a.nrhs + r) * K;
+        }
+    }
+    auto load = [&](int st, int k0) {
+        if constexpr (VA) {
+            const int k = k0 + (tid % 8) * 4;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int r = tid / 8 + 8 * i;
+                const bool in = m0 + r < M && k < kend;
+                sg_copy16(&As[st][r][(tid % 8) * 4], in ? A + (long)(m0 + r) * lda + k : A, in);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                // A^T: along the rows of the tile; A: along the depth
+                const int r = a.trans ? tid % 32 : tid / 32 + 2 * i, kk = a.trans ? tid / 32 + 2 * i : tid % 32;
+                const bool in = m0 + r < M && k0 + kk < kend;
+                const float* src = a.trans ? A + (long)(k0 + kk) * lda + m0 + r : A + (long)(m0 + r) * lda + k0 + kk;
+                sg_copy4(&As[st][r][kk], in ? src : A, in);
+            }
+        }
+        const int k = k0 + (tid % 8) * 4;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const bool in = bcol[i] && k < kend;
+            sg_copy16(&Bs[st][tid / 8 + 8 * i][(tid % 8) * 4], in ? bcol[i] + k : a.B, in);
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < SG_STAGES - 1; q++) {
+        if (q < steps) load(q, kb + q * SG_K);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+    for (int q = 0; q < steps; q++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(SG_STAGES - 2) : "memory");
+        __syncthreads();  // step q has landed, and every thread is done with step q - 1's stage
+        const int next = q + SG_STAGES - 1;
+        if (next < steps) load(next % SG_STAGES, kb + next * SG_K);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const int st = q % SG_STAGES;
+#pragma unroll
+        for (int k = 0; k < SG_K; k += 4) {
+            float4 x[4], y[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) x[i] = *reinterpret_cast<const float4*>(&As[st][tm + 8 * i][k]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) y[j] = *reinterpret_cast<const float4*>(&Bs[st][tn + 8 * j][k]);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    acc[i][j] = fmaf(x[i].x, y[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(x[i].y, y[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(x[i].z, y[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(x[i].w, y[j].w, acc[i][j]);
+                }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int c = col0 + tn + 8 * j;
+        if (c >= ncols) continue;
+        const int p = c / a.nrhs, r = c - p * a.nrhs;
+        float* d = a.D + ((long)a.out_cell[pair0 + p] * a.nrhs + r) * M;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int row = m0 + tm + 8 * i;
+            if (row >= M) continue;
+            if (a.mode == GEMM_STORE) d[row] = acc[i][j];
+            else if (a.mode == GEMM_ADD) d[row] += acc[i][j];
+            else atomicAdd(d + row, acc[i][j]);
+        }
+    }
 }
 
 // ---------------------------------------------------------------- FP64 GEMM

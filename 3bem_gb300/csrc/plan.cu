@@ -213,7 +213,14 @@ void GemmSet::run_rect(const T* B, T* D, int m, int k, int lda, int nrhs, int tr
     TBEM_CK(cudaGetDevice(&dev));
     TBEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     constexpr bool f64 = sizeof(T) == 8;
-    const int bn = f64 ? dgemm_bn(total_pairs() * nrhs, m, sms) : GM_BN;
+    // FP32 launches of fewer than two of the large tiles per SM: small tiles
+    // (a depth of a multiple of four)
+    const int bm0 = gemm_bm(m);
+    long big = 0;  // large tiles
+    if (!f64)
+        for (int np : npairs) big += ((long)np * nrhs + GM_BN - 1) / GM_BN * ((m + bm0 - 1) / bm0);
+    const bool small = !f64 && big < 2L * sms && k % 4 == 0;
+    const int bn = f64 ? dgemm_bn(total_pairs() * nrhs, m, sms) : small ? SG_B : GM_BN;
     const std::pair<int, int> key{nrhs, bn};
     auto it = tiles.find(key);
     if (it == tiles.end()) {
@@ -249,11 +256,11 @@ void GemmSet::run_rect(const T* B, T* D, int m, int k, int lda, int nrhs, int tr
     a.kchunk = k;
     const int nt = (int)it->second.first.n;
     if (nt == 0) return;
-    const int bm = f64 ? DG_ROWS * DG_WARPS : gemm_bm(m);
+    const int bm = f64 ? DG_ROWS * DG_WARPS : small ? SG_B : bm0;
     const int mt = (m + bm - 1) / bm;
-    const long ctas = (long)nt * mt;
-    // split K when the tiles fill less than two CTAs per SM and the
+    // split K when the (large) tiles fill less than two CTAs per SM and the
     // accumulation is atomic anyway (never for the deterministic modes)
+    const long ctas = f64 ? (long)nt * mt : big;
     int split = 1;
     if (mode == GEMM_ATOMIC && ctas < 2L * sms && k >= 128) {
         split = (int)std::min<long>(std::min<long>((2L * sms + ctas - 1) / ctas, 8), k / 64);
@@ -262,7 +269,10 @@ void GemmSet::run_rect(const T* B, T* D, int m, int k, int lda, int nrhs, int tr
     }
     const dim3 grid((unsigned)nt, (unsigned)mt, (unsigned)split);
     if constexpr (f64) dgemm_warp_kernel<<<grid, 32 * DG_WARPS, 0, s>>>(a, bn);
-    else if (bm == 128) grouped_gemm_kernel<128><<<grid, GM_THREADS, 0, s>>>(a);
+    else if (small) {
+        auto kern = !trans && lda % 4 == 0 ? small_gemm_kernel<true> : small_gemm_kernel<false>;
+        kern<<<grid, SG_THREADS, 0, s>>>(a);
+    } else if (bm == 128) grouped_gemm_kernel<128><<<grid, GM_THREADS, 0, s>>>(a);
     else grouped_gemm_kernel<64><<<grid, GM_THREADS, 0, s>>>(a);
     TBEM_CK(cudaGetLastError());
     if (launches) (*launches)++;
