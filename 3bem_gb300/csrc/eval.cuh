@@ -20,6 +20,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace tbem {
@@ -443,7 +445,7 @@ eval_kernel(const EvalArgs<T> a)
 // to all right-hand sides.  Sums as in eval_kernel (per tile in FP32, folded
 // into a compensated pair; TPT partial sums met by warp shuffles).
 template <int KID, bool TGT_SURF, int TPT, int WIDE>
-__global__ void __launch_bounds__(EVAL_THREADS / 2)
+__global__ void __launch_bounds__(EVAL_THREADS / 2, 7)
 eval_wide_kernel(const EvalArgs<float> a)
 {
     static_assert(kernel_dim(KID) == 1 && WIDE % 4 == 0, "scalar kernels, packed right-hand sides");
@@ -460,6 +462,9 @@ eval_wide_kernel(const EvalArgs<float> a)
     __shared__ Vec4<float> sl[SPLIT ? EVAL_THREADS : 1];
     __shared__ Vec4<float> snl[DF ? EVAL_THREADS : 1];
     __shared__ Vec4<float> sv[NV][EVAL_THREADS];
+    // the compensated sums, touched once per tile: in registers they left room
+    // for five CTAs per SM (a batch's near field of 64 right-hand sides 8.6 ms)
+    __shared__ float sacc[2][WIDE][NT], slo[2][WIDE][NT];
 
     const int task = a.item_task[blockIdx.x];
     const int t0 = a.item_start[blockIdx.x];
@@ -500,11 +505,14 @@ eval_wide_kernel(const EvalArgs<float> a)
         }
     }
 
-    float acc[2][WIDE], lo[2][WIDE], part[2][WIDE];
+    float part[2][WIDE];
 #pragma unroll
     for (int q = 0; q < 2; q++)
 #pragma unroll
-        for (int i = 0; i < WIDE; i++) { acc[q][i] = 0.f; lo[q][i] = 0.f; part[q][i] = 0.f; }
+        for (int i = 0; i < WIDE; i++) {
+            sacc[q][i][threadIdx.x] = slo[q][i][threadIdx.x] = 0.f;
+            part[q][i] = 0.f;
+        }
 
     const int b0 = a.task_src_ptr[task], b1 = a.task_src_ptr[task + 1];
     const int total = b1 > b0 ? a.src_blk_prefix[b1 - 1] + a.src_blk_count[b1 - 1] : 0;
@@ -547,7 +555,9 @@ eval_wide_kernel(const EvalArgs<float> a)
             }
         }
         __syncthreads();
-        if (act[0] || act[1]) {
+        // the pairs of this tile for the thread's first NQ targets
+        auto pairs = [&](auto targets) {
+            constexpr int NQ = decltype(targets)::value;
             const int n_here = min(EVAL_THREADS, total - tile);
             const float one[3] = {1.f, 0.f, 0.f};
             for (int j = lane; j < n_here; j += TPT) {
@@ -558,11 +568,11 @@ eval_wide_kernel(const EvalArgs<float> a)
                 if (DF && s.w != 0.f) {
                     const Vec4<float> nl = snl[j];
 #pragma unroll
-                    for (int q = 0; q < 2; q++)
+                    for (int q = 0; q < NQ; q++)
                         kv[q] = lapd_near_df(s, sq, nq, nl, px[q], py[q], pz[q], plx[q], ply[q], plz[q]);
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 2; q++) {
+                    for (int q = 0; q < NQ; q++) {
                         float dx = s.x - px[q], dy = s.y - py[q], dz = s.z - pz[q];
                         if (SPLIT) { dx += sq.x - plx[q]; dy += sq.y - ply[q]; dz += sq.z - plz[q]; }
                         accumulate<KID, false, float>(dx, dy, dz, pnx[q], pny[q], pnz[q], nq.x, nq.y,
@@ -573,7 +583,7 @@ eval_wide_kernel(const EvalArgs<float> a)
                 for (int r4 = 0; r4 < NV; r4++) {
                     const Vec4<float> vq = sv[r4][j];
 #pragma unroll
-                    for (int q = 0; q < 2; q++) {
+                    for (int q = 0; q < NQ; q++) {
                         part[q][4 * r4] += kv[q] * vq.x;
                         part[q][4 * r4 + 1] += kv[q] * vq.y;
                         part[q][4 * r4 + 2] += kv[q] * vq.z;
@@ -582,12 +592,32 @@ eval_wide_kernel(const EvalArgs<float> a)
                 }
             }
 #pragma unroll
-            for (int q = 0; q < 2; q++)
+            for (int q = 0; q < NQ; q++)
 #pragma unroll
-                for (int i = 0; i < WIDE; i++) { kahan_add(acc[q][i], lo[q][i], part[q][i]); part[q][i] = 0.f; }
+                for (int i = 0; i < WIDE; i++) {
+                    float hi = sacc[q][i][threadIdx.x], l = slo[q][i][threadIdx.x];
+                    kahan_add(hi, l, part[q][i]);
+                    sacc[q][i][threadIdx.x] = hi;
+                    slo[q][i][threadIdx.x] = l;
+                    part[q][i] = 0.f;
+                }
+        };
+        // a leaf's last CTA often holds no second targets at all
+        if (t0 + HALF < ntgt) {
+            if (act[0] || act[1]) pairs(std::integral_constant<int, 2>());
+        } else if (act[0]) {
+            pairs(std::integral_constant<int, 1>());
         }
         __syncthreads();
     }
+    float acc[2][WIDE], lo[2][WIDE];
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int i = 0; i < WIDE; i++) {
+            acc[q][i] = sacc[q][i][threadIdx.x];
+            lo[q][i] = slo[q][i][threadIdx.x];
+        }
     // the TPT partial sums of a target pair (consecutive lanes of one warp)
 #pragma unroll
     for (int off = TPT / 2; off > 0; off /= 2) {
