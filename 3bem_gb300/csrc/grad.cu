@@ -488,13 +488,13 @@ void Plan::source_gradients(const double* x, const double* r, double* g_y, doubl
     double* rt = grad_buf.p + off_r;
     double* out = grad_buf.p + off_o;
     double* gu = grad_buf.p + off_u;
-    apply(r, out, 1, s, true);  // r is in io_x now, the transposed states in cu / cd
+    apply(r, out, 1, s, true);  // r is at x_dev now, the transposed states in cu / cd
     // x to the device (io_y is free after the apply), then both to tree order
     TBEM_CK(cudaMemcpyAsync(io_y.p, x, sizeof(double) * R * NS, cudaMemcpyDefault, s));
     gather_rows_kernel<<<blocks_for(NS * R), 256, 0, s>>>(io_y.p, dsrc->perm.p, xt, NS, R);
     TBEM_CK(cudaGetLastError());
     if (NO > 0) {
-        gather_rows_kernel<<<blocks_for(NO * R), 256, 0, s>>>(io_x.p, dobs.perm.p, rt, NO, R);
+        gather_rows_kernel<<<blocks_for(NO * R), 256, 0, s>>>(x_dev, dobs.perm.p, rt, NO, R);
         TBEM_CK(cudaGetLastError());
     }
     TBEM_CK(cudaMemsetAsync(g7, 0, sizeof(double) * 7 * NS, s));
@@ -582,12 +582,12 @@ void Plan::observation_gradients(const double* x, const double* r, double* g_x, 
     double* gu = grad_buf.p + off_u;
     double* uck = grad_buf.p + off_c;
     double* qdn = grad_buf.p + off_q;
-    apply(x, out, 1, s, false);  // x is in io_x now, the states in cdc / the M2P buffers
+    apply(x, out, 1, s, false);  // x is at x_dev now, the states in cdc / the M2P buffers
     TBEM_CK(cudaMemcpyAsync(io_y.p, r, sizeof(double) * R * NO, cudaMemcpyDefault, s));
     gather_rows_kernel<<<blocks_for(NO * R), 256, 0, s>>>(io_y.p, dobs.perm.p, rt, NO, R);
     TBEM_CK(cudaGetLastError());
     if (NS > 0) {
-        gather_rows_kernel<<<blocks_for(NS * R), 256, 0, s>>>(io_x.p, dsrc->perm.p, xt, NS, R, dsrc->w.p);
+        gather_rows_kernel<<<blocks_for(NS * R), 256, 0, s>>>(x_dev, dsrc->perm.p, xt, NS, R, dsrc->w.p);
         TBEM_CK(cudaGetLastError());
     }
     // down-check potentials of the L2P leaves (V cdc), then their

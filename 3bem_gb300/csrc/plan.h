@@ -437,9 +437,10 @@ struct Plan {
     TaskSet p2m_t, p2p_t, m2p_t, p2l_t, l2p_t, m2l_fly_t;
     // work buffers
     int cap_rhs = 0;
-    DBuf<double> io_x, io_y;            // device staging of caller data (original order)
-    double* xin = nullptr;              // the current chunk of right-hand sides in io_x
-    double* yout = nullptr;             // and its outputs in io_y
+    DBuf<double> io_x, io_y;            // device staging of host data (original order)
+    const double* x_dev = nullptr;      // the apply's input: the caller's buffer or io_x
+    const double* xin = nullptr;        // its current chunk of right-hand sides
+    double* yout = nullptr;             // and that chunk's outputs
     int rhs_chunk(int nrhs) const;
     DBuf<double> s64, y64;              // strengths / outputs in tree order
     DBuf<float> s32;
