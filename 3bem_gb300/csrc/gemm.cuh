@@ -344,6 +344,24 @@ __global__ void __launch_bounds__(SG_THREADS) small_gemm_kernel(const GemmArgs<f
     }
 }
 
+// ----------------------------------------- FP32 products of one to four columns
+//
+// Between trees of different points almost every (level difference, offset)
+// class of the M2L has its own operator and one to four pairs: 1,382 classes
+// for 4,615 pairs at 6,144 sources and 4,096 observers.  Such a product reads
+// its operator once for two multiply-adds per value: HBM-bound, where a tensor
+// tile multiplies 64 columns for two and reads three bf16 planes (6 bytes per
+// value against 4).  few_gemm_kernel<P, R>: a warp takes R rows at a time, the
+// lanes their depths in P 16-byte pieces (the columns stay in registers), and
+// the row sums meet in a transposing butterfly.  few_gemm_t_kernel: a thread
+// per four columns of A, eight rows in flight, the rows split over blockIdx.y.
+// Both add atomically.  At those sizes (ranks 320 x 288; 1,053 of 1,382 classes,
+// 388 MB of operators) the geometry gradient, one product and one transposed
+// one, went from 3.80 to 3.45 ms; the tensor-core launches had taken 190 and
+// 223 us.
+constexpr int FEW_COLS = 4, FEW_THREADS = 128, FEW_ROWS = 64, FEW_SPLIT = 2;
+constexpr int FEW_MAX_K = 512;  // P <= 4
+
 // ---------------------------------------------------------------- FP64 GEMM
 //
 // GB300 issues two FP64 FMAs per SM and clock (1.25 TFLOP/s), so an FP64

@@ -204,6 +204,139 @@ __global__ void __launch_bounds__(32 * DG_WARPS) dgemm_warp_kernel(const GemmArg
     else dgemm_warp<4>(a, g, col0, ncols, m0, kb, kend);
 }
 
+// Sums v[i] over the lanes; lane l returns the sum of v[l % N]: each step halves
+// the values a lane still carries (31 shuffles for 32 sums instead of 160).
+template <int N>
+__device__ __forceinline__ float lane_sums(float (&v)[N], int lane)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (o >= N) {
+#pragma unroll
+            for (int i = 0; i < N; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+        } else {
+#pragma unroll
+            for (int i = 0; i < o; i++) {
+                const float keep = lane & o ? v[i + o] : v[i], send = lane & o ? v[i] : v[i + o];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+    }
+    return v[0];
+}
+
+template <int P, int R>
+__global__ void __launch_bounds__(FEW_THREADS) few_gemm_kernel(const GemmArgs<float> a)
+{
+    const int g = blockIdx.x, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int M = a.m, K = a.k, cols = a.g_npairs[g];
+    const long pair0 = a.g_pair0[g];
+    const float* __restrict__ A = a.A[g];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 b[FEW_COLS][P];  // depths 4 (lane + 32 p) .. + 3 of the columns
+#pragma unroll
+    for (int c = 0; c < FEW_COLS; c++)
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            const int k = 4 * (lane + 32 * p);
+            b[c][p] = c < cols && k < K
+                          ? *reinterpret_cast<const float4*>(a.B + (long)a.in_cell[pair0 + c] * K + k) : zero;
+        }
+    const int r_end = min(M, (int)(blockIdx.y + 1) * FEW_ROWS);
+    for (int r0 = blockIdx.y * FEW_ROWS + warp * R; r0 < r_end; r0 += R * (FEW_THREADS / 32)) {
+        float4 x[R][P];
+#pragma unroll
+        for (int r = 0; r < R; r++)
+#pragma unroll
+            for (int p = 0; p < P; p++) {
+                const int k = 4 * (lane + 32 * p);
+                x[r][p] = r0 + r < M && k < K ? __ldcs(reinterpret_cast<const float4*>(A + (long)(r0 + r) * a.lda + k)) : zero;
+            }
+        float v[FEW_COLS * R];
+#pragma unroll
+        for (int c = 0; c < FEW_COLS; c++)
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                float t = 0.f;
+#pragma unroll
+                for (int p = 0; p < P; p++)
+                    t += x[r][p].x * b[c][p].x + x[r][p].y * b[c][p].y + x[r][p].z * b[c][p].z + x[r][p].w * b[c][p].w;
+                v[c * R + r] = t;
+            }
+        const float sum = lane_sums(v, lane);
+        const int c = lane / R, row = r0 + lane % R;
+        if (c < cols && c < FEW_COLS && row < M) atomicAdd(a.D + (long)a.out_cell[pair0 + c] * M + row, sum);
+    }
+}
+
+__global__ void __launch_bounds__(FEW_THREADS) few_gemm_t_kernel(const GemmArgs<float> a)
+{
+    // op(A) = A^T: a.m columns of the stored A are the outputs, a.k its rows
+    __shared__ float z[FEW_COLS][FEW_MAX_K / FEW_SPLIT];
+    const int g = blockIdx.x, M = a.m, K = a.k, cols = a.g_npairs[g];
+    const long pair0 = a.g_pair0[g];
+    const float* __restrict__ A = a.A[g];
+    const int per = (K + FEW_SPLIT - 1) / FEW_SPLIT, k0 = blockIdx.y * per, k1 = min(K, k0 + per);
+    for (int e = threadIdx.x; e < FEW_COLS * per; e += FEW_THREADS) {
+        const int c = e / per, k = k0 + e % per;
+        z[c][e % per] = c < cols && k < k1 ? a.B[(long)a.in_cell[pair0 + c] * K + k] : 0.f;
+    }
+    __syncthreads();
+    // M / 4 quads of outputs; threads left over take every `step`-th row
+    const int nq = M / 4, step = max(1, FEW_THREADS / nq), phase = threadIdx.x / min(nq, FEW_THREADS);
+    if (phase >= step) return;
+    for (int q = threadIdx.x % min(nq, FEW_THREADS); q < nq; q += FEW_THREADS) {
+        float4 acc[FEW_COLS];
+#pragma unroll
+        for (int c = 0; c < FEW_COLS; c++) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int k = k0 + phase; k < k1; k += step) {
+            const float4 x = __ldcs(reinterpret_cast<const float4*>(A + (long)k * a.lda + 4 * q));
+#pragma unroll
+            for (int c = 0; c < FEW_COLS; c++) {
+                const float v = z[c][k - k0];
+                acc[c].x += v * x.x;
+                acc[c].y += v * x.y;
+                acc[c].z += v * x.z;
+                acc[c].w += v * x.w;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < FEW_COLS; c++) {
+            if (c >= cols) break;
+            atomicAdd(reinterpret_cast<float4*>(a.D + (long)a.out_cell[pair0 + c] * M + 4 * q), acc[c]);
+        }
+    }
+}
+
+// Products of groups of at most FEW_COLS pairs, one right-hand side, added
+// atomically; m and k multiples of four, k (trans: both) at most FEW_MAX_K.
+void GemmSet::run_few(const float* B, float* D, int m, int k, int lda, int trans, cudaStream_t s, long* launches)
+{
+    if (empty()) return;
+    GemmArgs<float> a{};
+    a.A = reinterpret_cast<const float* const*>(d_A);
+    a.g_pair0 = d_pair0;
+    a.g_npairs = d_npairs;
+    a.in_cell = d_in;
+    a.out_cell = d_out;
+    a.B = B;
+    a.D = D;
+    a.m = m;
+    a.k = k;
+    a.lda = lda;
+    const unsigned groups = (unsigned)npairs.size();
+    if (trans) few_gemm_t_kernel<<<dim3(groups, FEW_SPLIT), FEW_THREADS, 0, s>>>(a);
+    else {
+        const dim3 grid(groups, (m + FEW_ROWS - 1) / FEW_ROWS);
+        if (k <= 256) few_gemm_kernel<2, 8><<<grid, FEW_THREADS, 0, s>>>(a);
+        else if (k <= 384) few_gemm_kernel<3, 4><<<grid, FEW_THREADS, 0, s>>>(a);
+        else few_gemm_kernel<4, 4><<<grid, FEW_THREADS, 0, s>>>(a);
+    }
+    TBEM_CK(cudaGetLastError());
+    if (launches) (*launches)++;
+}
+
 template <typename T>
 void GemmSet::run_rect(const T* B, T* D, int m, int k, int lda, int nrhs, int trans, int mode,
                        cudaStream_t s, long* launches)
@@ -1130,8 +1263,10 @@ void Plan::autotune_tc()
     }
     G.tc_bn = best_bn;
     G.tc_bk = best_bk;
-    f.m2l_c_t.tc_bn = best_bn;
-    f.m2l_c_t.tc_bk = best_bk;
+    for (GemmSet* g : {&f.m2l_c_t, &f.m2l_many, &f.m2l_many_t}) {
+        g->tc_bn = best_bn;
+        g->tc_bk = best_bk;
+    }
     for (auto& g : f.m2m) { g.tc_bn = best_bn; g.tc_bk = best_bk; }
     for (auto& g : f.l2l) { g.tc_bn = best_bn; g.tc_bk = best_bk; }
 }
@@ -2400,6 +2535,19 @@ void Plan::build_compression(Form& F, const CompressionInput& in)
     };
     F.m2l_c = GemmSet();
     F.m2l_c_t = GemmSet();
+    F.m2l_few = GemmSet();
+    F.m2l_few_t = GemmSet();
+    F.m2l_many = GemmSet();
+    F.m2l_many_t = GemmSet();
+    // Groups of a few pairs leave the tensor cores where most groups are that
+    // small and their operators do not fit the L2 (129 MB): there they are read
+    // from memory once per product either way, 4 bytes a value against the
+    // planes' 6.  Smaller sets (a sphere of 960 points: 3 MB) stay with the
+    // others: their time is one launch.
+    long n_few = 0;
+    for (int np : F.m2l.npairs) n_few += np <= FEW_COLS;
+    F.split_few = !f64 && opt.m2l_path == 0 && 2 * n_few > (long)F.m2l.npairs.size() && ri % 4 == 0 &&
+                  ro % 4 == 0 && std::max(ri, ro) <= FEW_MAX_K && 4.0 * n_few * cc > 129e6;
     for (size_t g = 0; g < F.m2l.A_off.size(); g++) {
         std::vector<std::pair<int, int>> pr;
         for (long p = F.m2l.pair0[g]; p < F.m2l.pair0[g] + F.m2l.npairs[g]; p++)
@@ -2408,6 +2556,11 @@ void Plan::build_compression(Form& F, const CompressionInput& in)
         if (idx < 0) throw Error(TBEM_ERR_STATE, "M2L operator without a compressed copy");
         F.m2l_c.add_group(idx * cc, pr);
         F.m2l_c_t.add_group(idx * cc, swap_pairs(pr));
+        if (F.split_few) {
+            const bool few = pr.size() <= (size_t)FEW_COLS;
+            (few ? F.m2l_few : F.m2l_many).add_group(idx * cc, pr);
+            (few ? F.m2l_few_t : F.m2l_many_t).add_group(idx * cc, swap_pairs(pr));
+        }
     }
     // M2M / L2L per level and octant on the X / Y pools, pruned to the pairs
     // that reach a result: an upward state is used only if the cell or an
@@ -2508,6 +2661,8 @@ void Plan::build_compression(Form& F, const CompressionInput& in)
     };
     F.m2l_c.upload(pool(F.Cops, F.Cops64), es);
     F.m2l_c_t.upload(pool(F.Cops, F.Cops64), es);
+    if (F.split_few)
+        for (GemmSet* g : {&F.m2l_few, &F.m2l_many, &F.m2l_few_t, &F.m2l_many_t}) g->upload(F.Cops.p, es);
     for (auto& g : F.m2m_c) g.upload(pool(F.Xops, F.Xops64), es);
     for (auto& g : F.m2m_c_t) g.upload(pool(F.Xops, F.Xops64), es);
     for (auto& g : F.l2l_c) g.upload(pool(F.Yops, F.Yops64), es);
@@ -3023,10 +3178,15 @@ void Plan::forward_compressed(int nrhs, cudaStream_t s)
     bool tc_done = false;
     if constexpr (sizeof(T) == 4) {
         if (F.use_tc_c) {
-            F.tc_c.split_b_rows(cuc, 0, ncs * nrhs, std::max(ncs, nco) * nrhs, far);
-            launches++;
-            mark("m2l_split", far);
-            F.m2l_c.run_tc(F.tc_c, cdc, nrhs, 1, (long)ro * ri, far, &launches);
+            const bool few = F.split_few && nrhs == 1;
+            if (few) F.m2l_few.run_few(cuc, cdc, ro, ri, ri, 0, far, &launches);
+            GemmSet& G = few ? F.m2l_many : F.m2l_c;
+            if (!G.empty()) {
+                F.tc_c.split_b_rows(cuc, 0, ncs * nrhs, std::max(ncs, nco) * nrhs, far);
+                launches++;
+                mark("m2l_split", far);
+                G.run_tc(F.tc_c, cdc, nrhs, 1, (long)ro * ri, far, &launches);
+            }
             tc_done = true;
         }
     } else if (F.use_oz) {
@@ -3101,9 +3261,14 @@ void Plan::adjoint_compressed(int nrhs, cudaStream_t s)
     bool tc_done = false;
     if constexpr (sizeof(T) == 4) {
         if (F.use_tc_c) {
-            F.tc_c.split_b_rows(cdc, 0, nco * nrhs, std::max(ncs, nco) * nrhs, far, true);
-            launches++;
-            F.m2l_c_t.run_tc(F.tc_c, cuc, nrhs, 1, (long)ro * ri, far, &launches, true);
+            const bool few = F.split_few && nrhs == 1;
+            if (few) F.m2l_few_t.run_few(cdc, cuc, ri, ro, ri, 1, far, &launches);
+            GemmSet& G = few ? F.m2l_many_t : F.m2l_c_t;
+            if (!G.empty()) {
+                F.tc_c.split_b_rows(cdc, 0, nco * nrhs, std::max(ncs, nco) * nrhs, far, true);
+                launches++;
+                G.run_tc(F.tc_c, cuc, nrhs, 1, (long)ro * ri, far, &launches, true);
+            }
             tc_done = true;
         }
     }

@@ -305,6 +305,8 @@ struct GemmSet {
     // trans: op(A) = A^T (B from planes split with trans, D columns of P.k rows)
     void run_tc(const TcPlanes& P, float* D, int nrhs, int atomic, long nn, cudaStream_t s,
                 long* launches, bool trans = false);
+    // groups of at most FEW_COLS pairs, one right-hand side, in FP32 (gemm.cuh)
+    void run_few(const float* B, float* D, int m, int k, int lda, int trans, cudaStream_t s, long* launches);
     // FP64 products through the digit planes, added atomically into D
     std::map<int, DBuf<int4>> oz_tiles;  // per nrhs
     void run_oz(const OzPlanes& P, double* D, int nrhs, cudaStream_t s, long* launches);
@@ -394,6 +396,10 @@ struct Form {
     bool use_oz = false;
     DBuf<double> V64;  // V in FP64 (column-major n x r_out) while the L2P operators are built
     GemmSet m2l_c, m2l_c_t, comp_p2m, decomp_m2p, comp_p2l;
+    // precision form, one right-hand side: the M2L's groups of at most FEW_COLS
+    // pairs and the others, where most groups are that small (else empty)
+    GemmSet m2l_few, m2l_many, m2l_few_t, m2l_many_t;
+    bool split_few = false;
     GemmSet decomp_l2p;  // V over the L2P leaves: their down-check potentials (gradients)
     std::vector<GemmSet> c2e_l2p;  // per level: C2E_down over those leaves
     std::vector<GemmSet> m2m_c, m2m_c_t, l2l_c, l2l_c_t;  // per level

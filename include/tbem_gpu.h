@@ -96,7 +96,7 @@ typedef struct {
                               2 tcgen05 3xBF16 for the uncompressed M2L only,
                               3 tcgen05 3xBF16 for M2L, M2M and L2L,
                               4 SVD-compressed far field on the SIMT FP32 pipes,
-                              5 as 4 with the M2L products on tcgen05 3xBF16;
+                              5 as 4 with all M2L products on tcgen05 3xBF16;
                               FP64 compressed form: 4 the M2L on the FP64 pipe,
                               else through exact digit planes on tcgen05          */
     int p2p_block;         /* 0 auto; else threads per target in the P2P kernel (1,2,4,8) */
