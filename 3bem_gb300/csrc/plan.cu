@@ -2540,14 +2540,15 @@ void Plan::build_compression(Form& F, const CompressionInput& in)
     F.m2l_many = GemmSet();
     F.m2l_many_t = GemmSet();
     // Groups of a few pairs leave the tensor cores where most groups are that
-    // small and their operators do not fit the L2 (129 MB): there they are read
-    // from memory once per product either way, 4 bytes a value against the
-    // planes' 6.  Smaller sets (a sphere of 960 points: 3 MB) stay with the
-    // others: their time is one launch.
+    // small and their operators take 40 MB: measured (forward apply, tensor
+    // cores / from memory; most groups of a few pairs), 26 MB 82 / 87 us,
+    // 31 MB 87 / 89, 52 MB 150 / 123, 231 MB 184 / 138, 388 MB 379 / 269.
+    // Where the other groups are the majority (a closed surface's own tree:
+    // 1,220 of 2,788 classes hold 3 % of the pairs) the tiles stay.
     long n_few = 0;
     for (int np : F.m2l.npairs) n_few += np <= FEW_COLS;
     F.split_few = !f64 && opt.m2l_path == 0 && 2 * n_few > (long)F.m2l.npairs.size() && ri % 4 == 0 &&
-                  ro % 4 == 0 && std::max(ri, ro) <= FEW_MAX_K && 4.0 * n_few * cc > 129e6;
+                  ro % 4 == 0 && std::max(ri, ro) <= FEW_MAX_K && 4.0 * n_few * cc > 40e6;
     for (size_t g = 0; g < F.m2l.A_off.size(); g++) {
         std::vector<std::pair<int, int>> pr;
         for (long p = F.m2l.pair0[g]; p < F.m2l.pair0[g] + F.m2l.npairs[g]; p++)

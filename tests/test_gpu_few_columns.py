@@ -15,6 +15,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("kernel,size,n_obs,tol", [
     ("ElasticDisplacement", 32, 4096, 1e-7), ("ElasticDisplacement", 27, 1777, 1e-7), ("ElasticTraction", 30, 2500, 1e-7),
+    ("LaplaceSingle", 32, 4096, 1e-7),  # ranks below 128
     ("ElasticDisplacement", 24, 1500, 1e-8)])  # larger ranks: more pieces of a row per lane
 def test_small_groups_match_the_tensor_cores(kernel, size, n_obs, tol):
     from tbempy import ThreeD, meshes
