@@ -1311,6 +1311,7 @@ void Plan::autotune_p2p()
             float t = 0.f;
             TBEM_CK(cudaEventElapsedTime(&t, e0, e1));
             if (rep > 0) ms = std::min(ms, t);  // the first run warms the caches
+            if (rep > 1 && ms > 20.f) break;    // long launches repeat within the margin
         }
         if (ms < (mixed ? AUTOTUNE_MARGIN_FP32 : AUTOTUNE_MARGIN_FP64) * best) {
             best = ms;
@@ -1349,6 +1350,7 @@ void Plan::autotune_p2m()
             float t = 0.f;
             TBEM_CK(cudaEventElapsedTime(&t, e0, e1));
             if (rep > 0) ms = std::min(ms, t);
+            if (rep > 1 && ms > 20.f) break;
         }
         if (ms < (mixed ? AUTOTUNE_MARGIN_FP32 : AUTOTUNE_MARGIN_FP64) * best) {
             best = ms;
