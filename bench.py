@@ -892,9 +892,10 @@ def run_nearfield(args, rank, world, local):
     torch.cuda.synchronize()
     with ClockSampler(local) as clk:
         ms = _events_ms(torch, lambda: near.apply(xd), args.steps, stream, flush)
-    # algorithmic bytes of one apply: values and column indices once, row
-    # pointers, the output, and x once (a lower bound for the gathers)
-    algo = nnz * (8 + 8) + (rows + 1) * 8 + rows * 8 + cols * 8
+    # algorithmic bytes of one apply: values and column indices (kept in 32
+    # bits on the device) once, row pointers, the output, and x once (a lower
+    # bound for the gathers)
+    algo = nnz * (8 + 4) + (rows + 1) * 8 + rows * 8 + cols * 8
     hbm, _, peak_kind = peaks()
     achieved = algo / (ms / 1e3) / 1e9
     import scipy.sparse as sp

@@ -186,7 +186,7 @@ int tbem_fmm_apply_adjoint(TbemFmm* h, const double* z, double* w, int n_rhs, vo
  * (g_src_weights [n_src]); any output may be NULL.  One transposed apply of
  * r, then the three transposed passes that reach source points (near
  * field, points to up-check surfaces, points to down-check surfaces) again
- * with the kernel's exact derivatives (FP64 dual numbers), the far field
+ * with the kernel's exact derivatives (FP64, written out per kernel), the far field
  * entering through the transposed check-surface states of that apply
  * (recomputed per call, nothing stored).  The O(N) counterpart of
  * tbem_direct_gradients' source outputs for the compressed forms (precision
@@ -202,7 +202,7 @@ int tbem_fmm_source_gradients(TbemFmm* h, const double* x, const double* r, doub
  * One forward apply of x, then the three passes that reach observation
  * points (near field, M2P from the sources' up-equivalent surfaces, L2P from
  * the leaves' down-equivalent surfaces) again with the kernel's exact
- * derivatives (FP64 dual numbers); the down-equivalent densities are
+ * derivatives (FP64, written out per kernel); the down-equivalent densities are
  * rebuilt from the apply's compressed local coefficients.  The O(N)
  * counterpart of tbem_direct_gradients' observation outputs for the
  * compressed forms (TBEM_ERR_STATE for the plain and batched forms).
@@ -313,7 +313,7 @@ int tbem_direct_apply(int kernel, const double* kernel_params,
  * w_j K(x_i, y_j; n_i, n_j) and L = r^T A x it writes dL/d(obs_locs) [n_obs][3],
  * dL/d(obs_normals), dL/d(src_locs) [n_src][3], dL/d(src_normals),
  * dL/d(src_weights) [n_src] and dL/dx = A^T r [C][n_src].  Kernel derivatives
- * are exact (forward-mode dual numbers on the device).  Any output may be
+ * are exact (written out per kernel, FP64 on the device).  Any output may be
  * NULL; host or device memory. */
 int tbem_direct_gradients(int kernel, const double* kernel_params,
                           const double* obs_locs, const double* obs_normals, long n_obs,
