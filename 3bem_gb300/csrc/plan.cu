@@ -827,29 +827,29 @@ __global__ void __launch_bounds__(256) l2p_mixed_kernel(const float* E, const lo
 }
 
 // Its transpose: cd[leaf][r][k] = sum_rows E[row][k] z[r][d][pt0 + i], for NR
-// right-hand sides from r0.  HBM-bound on E: one CTA per leaf reads whole rows
-// in 16-byte pieces, a thread per piece of the row and as many row groups as
-// the CTA holds, four rows in flight per thread; the leaf's inputs sit in
-// shared memory and the row groups' sums meet there in a fixed order.  24,576
-// points, r_out 256 (E 78 MB): 45 us with a thread per column and a row at a
-// time, 27 us now.
-constexpr int L2PT_THREADS = 256, L2PT_ROWS = 128;
+// right-hand sides from r0.  Every sum is one chain over the leaf's rows in
+// their order, with a fused multiply-add per row: the transposed apply's FP32
+// results follow that order at 1e-8 (row groups summed side by side had moved
+// the transposed apply by up to seven times what its atomic sums repeat to).
+// HBM-bound on E: a thread owns 8 bytes of the row and reads L2PT_U rows ahead
+// of their multiply-adds, the leaf's inputs sit in shared memory (zero past the
+// last row).  24,576 points, r_out 256 (E 78 MB): 45 us with a thread per
+// column and a row at a time.
+constexpr int L2PT_THREADS = 256, L2PT_ROWS = 128, L2PT_U = 32;
 template <typename T, int NR>
 __global__ void __launch_bounds__(L2PT_THREADS) l2p_mixed_t_kernel(
     const T* E, const long* row0, const int* leaf, const long* pt0, const int* npts, const T* z, long z_n,
     int n, int ld, int R, int nrhs, int r0, T* cd)
 {
-    constexpr int V = 16 / (int)sizeof(T);
-    using Vec = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+    constexpr int V = 8 / (int)sizeof(T);
+    using Vec = typename std::conditional<sizeof(T) == 4, float2, double>::type;
     __shared__ T zs[NR][L2PT_ROWS];
-    __shared__ T red[L2PT_THREADS * V];
     const int t = blockIdx.x;
     const int rows = npts[t] * R;
     const T* Et = E + row0[t] * (long)ld;
     const int Q = (n + V - 1) / V;  // pieces of a row (the padding beyond n is zero)
-    for (int qb = 0; qb < Q; qb += L2PT_THREADS) {
-        const int nq = min(Q - qb, L2PT_THREADS), G = L2PT_THREADS / nq;
-        const int q = threadIdx.x % nq, g = threadIdx.x / nq;
+    for (int q0 = 0; q0 < Q; q0 += blockDim.x) {
+        const int q = q0 + threadIdx.x;
         T acc[NR][V];
 #pragma unroll
         for (int r = 0; r < NR; r++)
@@ -858,41 +858,36 @@ __global__ void __launch_bounds__(L2PT_THREADS) l2p_mixed_t_kernel(
         for (int rt = 0; rt < rows; rt += L2PT_ROWS) {
             const int nr = min(rows - rt, L2PT_ROWS);
             __syncthreads();
-            for (int e = threadIdx.x; e < nr * NR; e += L2PT_THREADS) {
-                const int r = e / nr, row = rt + e % nr;
-                zs[r][e % nr] = r0 + r < nrhs ? z[((long)(r0 + r) * R + row % R) * z_n + pt0[t] + row / R] : T(0);
+            for (int e = threadIdx.x; e < NR * L2PT_ROWS; e += blockDim.x) {
+                const int r = e / L2PT_ROWS, i = e % L2PT_ROWS, row = rt + i;
+                zs[r][i] = i < nr && r0 + r < nrhs ? z[((long)(r0 + r) * R + row % R) * z_n + pt0[t] + row / R] : T(0);
             }
             __syncthreads();
-            if (g >= G) continue;
-            const T* Eq = Et + (long)rt * ld + (qb + q) * V;
-#pragma unroll 4
-            for (int row = g; row < nr; row += G) {
-                const Vec w = __ldcs(reinterpret_cast<const Vec*>(Eq + (long)row * ld));
-                T v[V];
-                if constexpr (sizeof(T) == 4) { v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w; }
-                else { v[0] = w.x; v[1] = w.y; }
+            if (q >= Q) continue;
+            const T* Eq = Et + (long)rt * ld + (long)q * V;
+            for (int b = 0; b < nr; b += L2PT_U) {
+                Vec w[L2PT_U];
 #pragma unroll
-                for (int r = 0; r < NR; r++)
+                for (int u = 0; u < L2PT_U; u++)
+                    w[u] = b + u < nr ? __ldcs(reinterpret_cast<const Vec*>(Eq + (long)(b + u) * ld)) : Vec{};
 #pragma unroll
-                    for (int c = 0; c < V; c++) acc[r][c] += v[c] * zs[r][row];
-            }
-        }
+                for (int u = 0; u < L2PT_U; u++) {
+                    T v[V];
+                    if constexpr (V == 2) { v[0] = w[u].x; v[1] = w[u].y; }
+                    else v[0] = w[u];
 #pragma unroll
-        for (int r = 0; r < NR; r++) {
-            __syncthreads();
-            if (g < G)
+                    for (int r = 0; r < NR; r++)
 #pragma unroll
-                for (int c = 0; c < V; c++) red[(g * nq + q) * V + c] = acc[r][c];
-            __syncthreads();
-            if (r0 + r < nrhs)
-                for (int e = threadIdx.x; e < nq * V; e += L2PT_THREADS) {
-                    const int k = qb * V + e;
-                    if (k >= n) continue;
-                    T v = T(0);
-                    for (int gg = 0; gg < G; gg++) v += red[gg * nq * V + e];
-                    cd[((long)leaf[t] * nrhs + r0 + r) * n + k] = v;
+                        for (int c = 0; c < V; c++) acc[r][c] += v[c] * zs[r][b + u];
                 }
+            }
         }
+        if (q >= Q) continue;
+#pragma unroll
+        for (int r = 0; r < NR; r++)
+#pragma unroll
+            for (int c = 0; c < V; c++)
+                if (r0 + r < nrhs && q * V + c < n) cd[((long)leaf[t] * nrhs + r0 + r) * n + q * V + c] = acc[r][c];
     }
 }
 
@@ -1263,10 +1258,8 @@ void Plan::autotune_tc()
     }
     G.tc_bn = best_bn;
     G.tc_bk = best_bk;
-    for (GemmSet* g : {&f.m2l_c_t, &f.m2l_many, &f.m2l_many_t}) {
-        g->tc_bn = best_bn;
-        g->tc_bk = best_bk;
-    }
+    f.m2l_many.tc_bn = best_bn;
+    f.m2l_many.tc_bk = best_bk;
     for (auto& g : f.m2m) { g.tc_bn = best_bn; g.tc_bk = best_bk; }
     for (auto& g : f.l2l) { g.tc_bn = best_bn; g.tc_bk = best_bk; }
 }
@@ -2780,10 +2773,11 @@ void Plan::launch_l2p_t(const T* z, int len, int nrhs, T* cd, cudaStream_t s)
     Form& F = f;
     const T* E;
     if constexpr (sizeof(T) == 4) E = F.E.p; else E = F.E64.p;
+    const int pieces = (int)((len * sizeof(T) + 7) / 8), threads = std::min(L2PT_THREADS, (pieces + 31) / 32 * 32);
     for (int r0 = 0; r0 < nrhs;) {
         const bool one = nrhs - r0 == 1;
         auto kern = one ? l2p_mixed_t_kernel<T, 1> : l2p_mixed_t_kernel<T, 4>;
-        kern<<<F.n_l2p, L2PT_THREADS, 0, s>>>(E, F.E_row0.p, F.E_leaf.p, F.E_pt0.p, F.E_npts.p, z, n_obs, len,
+        kern<<<F.n_l2p, threads, 0, s>>>(E, F.E_row0.p, F.E_leaf.p, F.E_pt0.p, F.E_npts.p, z, n_obs, len,
                                               F.E_ld, R, nrhs, r0, cd);
         TBEM_CK(cudaGetLastError());
         launches++;
@@ -3260,22 +3254,17 @@ void Plan::adjoint_compressed(int nrhs, cudaStream_t s)
     eval<T>(p2p_t, kid, false, false, S, *dsrc, 0, dobs, 0, zin, NO, nullptr, s64.p, NS, nullptr, 1, nrhs, near, true);
     for (int l = O.n_levels() - 1; l >= 1; l--)
         if (l - 1 < (int)F.l2l_c_t.size()) F.l2l_c_t[l - 1].run_rect<T>(cdc, cdc, ro, ro, ro, nrhs, 1, GEMM_ATOMIC, far, &launches);
-    // C_k^T on the tensor cores from the forward planes, as the forward M2L
-    bool tc_done = false;
+    // C_k^T in multiply-adds of the form's precision.  The forward planes on
+    // the tensor cores (three bf16 terms, accumulators that truncate) took the
+    // whole apply from 497 to 277 us (24,576 points, traction), but moved its
+    // results by four to five times what calls differ by and added 1 to 2 % to
+    // their error against FP64 (18 operators).
+    bool few = false;
     if constexpr (sizeof(T) == 4) {
-        if (F.use_tc_c) {
-            const bool few = F.split_few && nrhs == 1;
-            if (few) F.m2l_few_t.run_few(cdc, cuc, ri, ro, ri, 1, far, &launches);
-            GemmSet& G = few ? F.m2l_many_t : F.m2l_c_t;
-            if (!G.empty()) {
-                F.tc_c.split_b_rows(cdc, 0, nco * nrhs, std::max(ncs, nco) * nrhs, far, true);
-                launches++;
-                G.run_tc(F.tc_c, cuc, nrhs, 1, (long)ro * ri, far, &launches, true);
-            }
-            tc_done = true;
-        }
+        few = F.use_tc_c && F.split_few && nrhs == 1;
+        if (few) F.m2l_few_t.run_few(cdc, cuc, ri, ro, ri, 1, far, &launches);
     }
-    if (!tc_done) F.m2l_c_t.run_rect<T>(cdc, cuc, ri, ro, ri, nrhs, 1, GEMM_ATOMIC, far, &launches);
+    (few ? F.m2l_many_t : F.m2l_c_t).run_rect<T>(cdc, cuc, ri, ro, ri, nrhs, 1, GEMM_ATOMIC, far, &launches);
     if (!L.p2l.empty()) {
         F.comp_p2l.run_rect<T>(cdc, cd, n, ro, ro, nrhs, 0, GEMM_STORE, far, &launches);
     }

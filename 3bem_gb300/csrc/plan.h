@@ -245,11 +245,9 @@ struct TcPlanes {
     DBuf<int> err;  // set by a tensor-core GEMM whose bounded wait gave up
     long long wait_cycles = 0;  // budget of the GEMM's bounded waits (0: the default)
     void build(const float* ops32, long n_ops, int m, int k, cudaStream_t s);
-    // split rows [row0, row0 + rows) of a [rows_total][k] buffer (trans: [m],
-    // the B operand of A^T) into the same rows of the planes (capacity for
-    // rows_total rows)
-    void split_b_rows(const float* cells, long row0, long rows, long rows_total, cudaStream_t s,
-                      bool trans = false);
+    // split rows [row0, row0 + rows) of a [rows_total][k] buffer into the same
+    // rows of the planes (capacity for rows_total rows)
+    void split_b_rows(const float* cells, long row0, long rows, long rows_total, cudaStream_t s);
 };
 
 // Digit planes of the FP64 compressed form's M2L operators for the tensor-core
@@ -302,9 +300,8 @@ struct GemmSet {
     std::map<int, TcTiles> tc_tiles;  // per (nrhs, N tile)
     int tc_bn = 128;  // N tile of the tensor-core path (128 or 64; autotuned)
     int tc_bk = 64;   // K chunk (64, or 32 with N = 128; autotuned)
-    // trans: op(A) = A^T (B from planes split with trans, D columns of P.k rows)
     void run_tc(const TcPlanes& P, float* D, int nrhs, int atomic, long nn, cudaStream_t s,
-                long* launches, bool trans = false);
+                long* launches);
     // groups of at most FEW_COLS pairs, one right-hand side, in FP32 (gemm.cuh)
     void run_few(const float* B, float* D, int m, int k, int lda, int trans, cudaStream_t s, long* launches);
     // FP64 products through the digit planes, added atomically into D

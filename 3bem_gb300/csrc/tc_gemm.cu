@@ -79,8 +79,7 @@ constexpr int TC_THREADS_P = TC_EPILOGUE + TC_PRODUCERS + 32;  // epilogue + pro
 struct TcArgs {
     const __nv_bfloat16* A[TC_TERMS];  // [op][m_pad][k_pad] per term
     long a_op_stride;                  // m_pad * k_pad
-    int a_ld;                          // row length of the stored operators (k_pad)
-    int k_len;                         // depth of the product: k_pad, or m padded to 64 for A^T
+    int k_pad;
     // per column tile: {operator, first pair of its group, first column of
     // the tile within the group, columns of the group}; column c of a group
     // is (pair pair0 + c / nrhs, right-hand side c % nrhs), its B row
@@ -93,7 +92,7 @@ struct TcArgs {
     const int* in_cell;
     const int* out_cell;
     int nrhs;
-    const __nv_bfloat16* B[TC_TERMS];  // [cell][rhs][k_len] per term
+    const __nv_bfloat16* B[TC_TERMS];  // [cell][rhs][k_pad] per term
     float* D;                          // [cell][rhs][n]
     int n;
     int atomic;
@@ -103,10 +102,7 @@ struct TcArgs {
 
 namespace {
 
-// TRANS: op(A) = A^T, read from the same planes.  A stage then holds BK rows of
-// A (the depth) by 128 of its columns (the output rows), and the MMA takes it
-// as an MN-major operand.
-template <int BN, int BK, bool TRANS>
+template <int BN, int BK>
 __global__ void __launch_bounds__(TC_THREADS_P, 1) tc_gemm_kernel(const TcArgs a, int n_ctiles, int m_tiles)
 {
     using Sh = TcShape<BN, BK>;
@@ -122,7 +118,7 @@ __global__ void __launch_bounds__(TC_THREADS_P, 1) tc_gemm_kernel(const TcArgs a
     uint8_t* smem = reinterpret_cast<uint8_t*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const int nk = a.k_len / BK;
+    const int nk = a.k_pad / BK;
     const int total = n_ctiles * m_tiles;
 
     if (warp == 0) {
@@ -198,15 +194,10 @@ __global__ void __launch_bounds__(TC_THREADS_P, 1) tc_gemm_kernel(const TcArgs a
         bool ok = true;
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
             const int m0 = (t % m_tiles) * TC_BM;
-            // TRANS: 16 pieces per depth row, depth rows pt / 16 + 8 i; columns
-            // past the stored row are zero-filled
-            const int tp = pt % 16, trow = pt / 16;
-            const bool tvalid = m0 + tp * 8 < a.a_ld;
-            const long a_base = (long)nop * a.a_op_stride +
-                                (TRANS ? (long)trow * a.a_ld + m0 + tp * 8 : (long)(m0 + prow) * a.a_ld + pj * 8);
+            const long a_base = (long)nop * a.a_op_stride + (long)(m0 + prow) * a.k_pad + pj * 8;
             long boff[B_PER];
 #pragma unroll
-            for (int i = 0; i < B_PER; i++) boff[i] = nb[i] >= 0 ? (long)nb[i] * a.k_len + pj * 8 : -1;
+            for (int i = 0; i < B_PER; i++) boff[i] = nb[i] >= 0 ? (long)nb[i] * a.k_pad + pj * 8 : -1;
             if (t + (int)gridDim.x < total) prefetch(t + gridDim.x);
             for (int kc = 0; kc < nk; kc++, j++) {
                 const int s = j % STAGES;
@@ -218,25 +209,12 @@ __global__ void __launch_bounds__(TC_THREADS_P, 1) tc_gemm_kernel(const TcArgs a
                 const int k0 = kc * BK;
 #pragma unroll
                 for (int q = 0; q < TC_TERMS; q++) {
-                    if constexpr (TRANS) {
 #pragma unroll
-                        for (int i = 0; i < BK / 8; i++) {
-                            const int row = trow + 8 * i;
-                            const uint32_t dst = st + q * Sh::A_TILE + (tp / 8) * (BK * 128) + row * 128 +
-                                                 (((tp % 8) ^ (row & 7)) << 4);
-                            const __nv_bfloat16* src = tvalid ? a.A[q] + a_base + (long)(k0 + 8 * i) * a.a_ld : a.A[q];
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
-                                         "r"(tvalid ? 16u : 0u)
-                                         : "memory");
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < A_PER; i++) {
-                            const int row = prow + RSTEP * i;
-                            const uint32_t dst = st + q * Sh::A_TILE + row * RB + (sw_piece<RB>(row, pj) << 4);
-                            const __nv_bfloat16* src = a.A[q] + a_base + (long)RSTEP * i * a.a_ld + k0;
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-                        }
+                    for (int i = 0; i < A_PER; i++) {
+                        const int row = prow + RSTEP * i;
+                        const uint32_t dst = st + q * Sh::A_TILE + row * RB + (sw_piece<RB>(row, pj) << 4);
+                        const __nv_bfloat16* src = a.A[q] + a_base + (long)RSTEP * i * a.k_pad + k0;
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
                     }
 #pragma unroll
                     for (int i = 0; i < B_PER; i++) {
@@ -289,22 +267,16 @@ __global__ void __launch_bounds__(TC_THREADS_P, 1) tc_gemm_kernel(const TcArgs a
 #pragma unroll
                     for (int kk = 0; kk < BK / 16; kk++) {
                         const uint32_t off = kk * 32;  // 16 bf16 along K inside the swizzle atom
-                        const uint32_t aoff = TRANS ? kk * 2048 : off;  // or 16 depth rows
+                        const uint32_t a0 = st + off, a1 = a0 + Sh::A_TILE, a2 = a0 + 2 * Sh::A_TILE;
                         const uint32_t b0 = st + B_BASE + off, b1 = b0 + Sh::B_TILE, b2 = b0 + 2 * Sh::B_TILE;
-                        auto a_desc = [&](int q) {
-                            const uint32_t p = st + aoff + q * Sh::A_TILE;
-                            if constexpr (TRANS) return mn_desc<BK>(p);
-                            else return sw_desc<RB>(p);
-                        };
-                        // bit 15: A is MN-major
-                        constexpr uint32_t ID = Sh::IDESC | (TRANS ? 1u << 15 : 0u);
+                        constexpr uint32_t ID = Sh::IDESC;
                         const uint32_t acc = (kc | kk) != 0;
-                        mma_bf16(big, a_desc(0), sw_desc<RB>(b0), ID, acc);
-                        mma_bf16(small, a_desc(0), sw_desc<RB>(b1), ID, acc);
-                        mma_bf16(small, a_desc(1), sw_desc<RB>(b0), ID, 1);
-                        mma_bf16(small, a_desc(0), sw_desc<RB>(b2), ID, 1);
-                        mma_bf16(small, a_desc(1), sw_desc<RB>(b1), ID, 1);
-                        mma_bf16(small, a_desc(2), sw_desc<RB>(b0), ID, 1);
+                        mma_bf16(big, sw_desc<RB>(a0), sw_desc<RB>(b0), ID, acc);
+                        mma_bf16(small, sw_desc<RB>(a0), sw_desc<RB>(b1), ID, acc);
+                        mma_bf16(small, sw_desc<RB>(a1), sw_desc<RB>(b0), ID, 1);
+                        mma_bf16(small, sw_desc<RB>(a0), sw_desc<RB>(b2), ID, 1);
+                        mma_bf16(small, sw_desc<RB>(a1), sw_desc<RB>(b1), ID, 1);
+                        mma_bf16(small, sw_desc<RB>(a2), sw_desc<RB>(b0), ID, 1);
                     }
                     mma_issued = true;
                     mma_commit(smem_u32(&empty_bar[s]));
@@ -435,32 +407,27 @@ void TcPlanes::build(const float* ops32, long n_ops, int m, int k, cudaStream_t 
     auto opt_in = [](auto kern, int bytes) {
         TBEM_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     };
-    opt_in(tc_gemm_kernel<128, 64, false>, TcShape<128, 64>::SMEM_BYTES);
-    opt_in(tc_gemm_kernel<64, 64, false>, TcShape<64, 64>::SMEM_BYTES);
-    opt_in(tc_gemm_kernel<128, 32, false>, TcShape<128, 32>::SMEM_BYTES);
-    opt_in(tc_gemm_kernel<256, 32, false>, TcShape<256, 32>::SMEM_BYTES);
-    opt_in(tc_gemm_kernel<128, 64, true>, TcShape<128, 64>::SMEM_BYTES);
-    opt_in(tc_gemm_kernel<64, 64, true>, TcShape<64, 64>::SMEM_BYTES);
-    opt_in(tc_gemm_kernel<128, 32, true>, TcShape<128, 32>::SMEM_BYTES);
-    opt_in(tc_gemm_kernel<256, 32, true>, TcShape<256, 32>::SMEM_BYTES);
+    opt_in(tc_gemm_kernel<128, 64>, TcShape<128, 64>::SMEM_BYTES);
+    opt_in(tc_gemm_kernel<64, 64>, TcShape<64, 64>::SMEM_BYTES);
+    opt_in(tc_gemm_kernel<128, 32>, TcShape<128, 32>::SMEM_BYTES);
+    opt_in(tc_gemm_kernel<256, 32>, TcShape<256, 32>::SMEM_BYTES);
 }
 
 void TcPlanes::split_b_rows(const float* cells, long row0, long rows, long rows_total,
-                            cudaStream_t s, bool trans)
+                            cudaStream_t s)
 {
-    const int len = trans ? m : k, len_pad = (len + TC_BK - 1) / TC_BK * TC_BK;
-    for (auto& p : b) p.ensure(std::max<long>(rows_total * (long)len_pad, 1));
-    const long total = rows * (long)len_pad;
+    for (auto& p : b) p.ensure(std::max<long>(rows_total * (long)k_pad, 1));
+    const long total = rows * (long)k_pad;
     if (total > 0) {
         split_rows_kernel<<<(unsigned)std::min<long>((total + 255) / 256, 152L * 64), 256, 0, s>>>(
-            cells + row0 * (long)len, rows, len, len_pad, b[0].p + row0 * len_pad, b[1].p + row0 * len_pad,
-            b[2].p + row0 * len_pad);
+            cells + row0 * (long)k, rows, k, k_pad, b[0].p + row0 * k_pad, b[1].p + row0 * k_pad,
+            b[2].p + row0 * k_pad);
         TBEM_CK(cudaGetLastError());
     }
 }
 
 void GemmSet::run_tc(const TcPlanes& P, float* D, int nrhs, int atomic, long nn, cudaStream_t s,
-                     long* launches, bool trans)
+                     long* launches)
 {
     if (empty()) return;
     // the autotuned N tile is one right-hand side's; with several, groups whose
@@ -508,8 +475,7 @@ void GemmSet::run_tc(const TcPlanes& P, float* D, int nrhs, int atomic, long nn,
         a.B[t] = P.b[t].p;
     }
     a.a_op_stride = (long)P.m_pad * P.k_pad;
-    a.a_ld = P.k_pad;
-    a.k_len = trans ? (P.m + TC_BK - 1) / TC_BK * TC_BK : P.k_pad;
+    a.k_pad = P.k_pad;
     a.tiles = it->second.t.p;
     a.tile_brow = it->second.brow.p;
     a.tile_drow = it->second.drow.p;
@@ -517,11 +483,11 @@ void GemmSet::run_tc(const TcPlanes& P, float* D, int nrhs, int atomic, long nn,
     a.out_cell = d_out;
     a.nrhs = nrhs;
     a.D = D;
-    a.n = trans ? P.k : P.m;
+    a.n = P.m;
     a.atomic = atomic;
     a.err = P.err.p;
     a.wait_cycles = P.wait_cycles > 0 ? P.wait_cycles : TC_WAIT_CYCLES;
-    const int n_ctiles = it->second.n, m_tiles = (a.n + TC_BM - 1) / TC_BM;
+    const int n_ctiles = it->second.n, m_tiles = P.m_pad / TC_BM;
     const long total = (long)n_ctiles * m_tiles;
     if (total == 0) return;
     int dev = 0, sms = 0;
@@ -529,13 +495,10 @@ void GemmSet::run_tc(const TcPlanes& P, float* D, int nrhs, int atomic, long nn,
     TBEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const unsigned grid = (unsigned)std::min<long>(total, std::max(sms, 1));
     auto go = [&](auto kern, int smem) { kern<<<grid, TC_THREADS_P, smem, s>>>(a, n_ctiles, m_tiles); };
-    if (bn == 64) go(trans ? tc_gemm_kernel<64, 64, true> : tc_gemm_kernel<64, 64, false>, TcShape<64, 64>::SMEM_BYTES);
-    else if (bn == 256)
-        go(trans ? tc_gemm_kernel<256, 32, true> : tc_gemm_kernel<256, 32, false>, TcShape<256, 32>::SMEM_BYTES);
-    else if (tc_bk == 32 && !wide)
-        go(trans ? tc_gemm_kernel<128, 32, true> : tc_gemm_kernel<128, 32, false>, TcShape<128, 32>::SMEM_BYTES);
-    else
-        go(trans ? tc_gemm_kernel<128, 64, true> : tc_gemm_kernel<128, 64, false>, TcShape<128, 64>::SMEM_BYTES);
+    if (bn == 64) go(tc_gemm_kernel<64, 64>, TcShape<64, 64>::SMEM_BYTES);
+    else if (bn == 256) go(tc_gemm_kernel<256, 32>, TcShape<256, 32>::SMEM_BYTES);
+    else if (tc_bk == 32 && !wide) go(tc_gemm_kernel<128, 32>, TcShape<128, 32>::SMEM_BYTES);
+    else go(tc_gemm_kernel<128, 64>, TcShape<128, 64>::SMEM_BYTES);
     TBEM_CK(cudaGetLastError());
     if (launches) (*launches)++;
 }

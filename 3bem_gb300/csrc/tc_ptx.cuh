@@ -27,21 +27,6 @@ __device__ __forceinline__ uint64_t sw_desc(uint32_t saddr)
     return d;
 }
 
-// The same for a tile stored depth-major (the A^T operand: BK depth rows of
-// 128 output rows): 64-wide column atoms of 128-byte rows with the 128-byte
-// swizzle, the atoms BK * 128 bytes apart, groups of eight depths 1024 bytes.
-template <int BK>
-__device__ __forceinline__ uint64_t mn_desc(uint32_t saddr)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
-    d |= (uint64_t)((BK * 128) >> 4) << 16;  // leading byte offset: next 64 rows of the output
-    d |= (uint64_t)(1024 >> 4) << 32;        // stride byte offset: next eight depths
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;                  // SWIZZLE_128B
-    return d;
-}
-
 // Position of 16-byte piece j of tile row r under the RB-byte swizzle: the
 // piece index XOR the row's position inside the 1024-byte (128B) or
 // 512-byte (64B) swizzle atom.
