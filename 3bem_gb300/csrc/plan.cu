@@ -1266,12 +1266,39 @@ void Plan::autotune_tc()
 
 namespace {
 // A timed variant replaces the best one so far only when it is faster by more
-// than repeated timings differ: variants that tie would otherwise fall either
-// way from one construction to the next, and with them the summation order,
-// which the plain form's pseudo-inverses turn into 1e-8 of the result (its
-// points-to-check-surface pass with 2 and 4 threads per target: 98.9 to 102 us
-// each on 15,360 points).
-constexpr float AUTOTUNE_MARGIN_FP32 = 0.995f, AUTOTUNE_MARGIN_FP64 = 0.97f;
+// than repeated timings differ (0.3 % for the FP32 passes, up to 3 % for the
+// FP64 ones, over four constructions of 40 operators): variants that tie would
+// otherwise fall either way from one construction to the next, and with them
+// the summation order, which shows in the results (points to check surfaces in
+// the plain form: its pseudo-inverses turn it into 1e-8; the FP32 near field:
+// 3e-7).
+constexpr float AUTOTUNE_MARGIN_FP32 = 0.99f, AUTOTUNE_MARGIN_FP64 = 0.97f;
+
+// Time of one launch of `run` on `s`, in ms.  Passes of small operators last
+// 6 to 50 us, of which an event pair resolves half a percent, and a lone
+// launch's own jitter is several: each sample is a row of launches of
+// AUTOTUNE_SPAN ms in all, and the fastest of four samples counts.  Launches
+// of 20 ms and more repeat within the margin and are timed twice.
+constexpr float AUTOTUNE_SPAN = 0.3f;
+template <typename F>
+float time_launch(cudaEvent_t e0, cudaEvent_t e1, cudaStream_t s, F&& run)
+{
+    auto row = [&](int n) {
+        TBEM_CK(cudaEventRecord(e0, s));
+        for (int i = 0; i < n; i++) run();
+        TBEM_CK(cudaEventRecord(e1, s));
+        TBEM_CK(cudaEventSynchronize(e1));
+        float t = 0.f;
+        TBEM_CK(cudaEventElapsedTime(&t, e0, e1));
+        return t / n;
+    };
+    row(1);  // warms the caches
+    float best = row(1);
+    const int n = (int)std::min(32.f, std::max(1.f, std::ceil(AUTOTUNE_SPAN / std::max(best, 1e-3f))));
+    if (n > 1) best = 1e30f;  // a lone launch is no sample of a row
+    for (int rep = 0; rep < (best > 20.f && n == 1 ? 1 : 4); rep++) best = std::min(best, row(n));
+    return best;
+}
 }  // namespace
 
 // Picks the point-to-point pass's threads per target (2, 4 or 8) by timing
@@ -1285,33 +1312,21 @@ void Plan::autotune_p2p()
     if (mixed) TBEM_CK(cudaMemsetAsync(s32.p, 0, sizeof(float) * R * n_src, stream));
     else TBEM_CK(cudaMemsetAsync(s64.p, 0, sizeof(double) * R * n_src, stream));
     ScopedEvent t0, t1;
-    const cudaEvent_t e0 = t0.e, e1 = t1.e;
     float best = 1e30f;
-    int best_tpt = 4;
     for (int tpt : {4, 2, 8}) {
-        p2p_tpt = tpt;
-        float ms = 1e30f;
-        for (int rep = 0; rep < 5; rep++) {
-            TBEM_CK(cudaEventRecord(e0, stream));
+        const float ms = time_launch(t0.e, t1.e, stream, [&] {
             if (mixed)
                 eval<float>(p2p, kid, false, false, otree, dobs, 0, *dsrc, 0, s32.p, n_src,
-                            nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, p2p_tpt);
+                            nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, tpt);
             else
                 eval<double>(p2p, kid, false, false, otree, dobs, 0, *dsrc, 0, s64.p, n_src,
-                             nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, p2p_tpt);
-            TBEM_CK(cudaEventRecord(e1, stream));
-            TBEM_CK(cudaEventSynchronize(e1));
-            float t = 0.f;
-            TBEM_CK(cudaEventElapsedTime(&t, e0, e1));
-            if (rep > 0) ms = std::min(ms, t);  // the first run warms the caches
-            if (rep > 1 && ms > 20.f) break;    // long launches repeat within the margin
-        }
+                             nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, tpt);
+        });
         if (ms < (mixed ? AUTOTUNE_MARGIN_FP32 : AUTOTUNE_MARGIN_FP64) * best) {
             best = ms;
-            best_tpt = tpt;
+            p2p_tpt = tpt;
         }
     }
-    p2p_tpt = best_tpt;
 }
 
 // Picks the points-to-check-surface pass's threads per target (1, 2 or 4)
@@ -1324,33 +1339,21 @@ void Plan::autotune_p2m()
     if (mixed) TBEM_CK(cudaMemsetAsync(s32.p, 0, sizeof(float) * R * n_src, stream));
     else TBEM_CK(cudaMemsetAsync(s64.p, 0, sizeof(double) * R * n_src, stream));
     ScopedEvent t0, t1;
-    const cudaEvent_t e0 = t0.e, e1 = t1.e;
     float best = 1e30f;
-    int best_tpt = 4;
     for (int tpt : {4, 2, 1}) {
-        p2m_tpt = tpt;
-        float ms = 1e30f;
-        for (int rep = 0; rep < 5; rep++) {
-            TBEM_CK(cudaEventRecord(e0, stream));
+        const float ms = time_launch(t0.e, t1.e, stream, [&] {
             if (mixed)
                 eval<float>(p2m, f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s32.p, n_src,
-                            nullptr, nullptr, 0, cu32.p, 0, 1, stream, false, p2m_tpt);
+                            nullptr, nullptr, 0, cu32.p, 0, 1, stream, false, tpt);
             else
                 eval<double>(p2m, f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s64.p, n_src,
-                             nullptr, nullptr, 0, cu64.p, 0, 1, stream, false, p2m_tpt);
-            TBEM_CK(cudaEventRecord(e1, stream));
-            TBEM_CK(cudaEventSynchronize(e1));
-            float t = 0.f;
-            TBEM_CK(cudaEventElapsedTime(&t, e0, e1));
-            if (rep > 0) ms = std::min(ms, t);
-            if (rep > 1 && ms > 20.f) break;
-        }
+                             nullptr, nullptr, 0, cu64.p, 0, 1, stream, false, tpt);
+        });
         if (ms < (mixed ? AUTOTUNE_MARGIN_FP32 : AUTOTUNE_MARGIN_FP64) * best) {
             best = ms;
-            best_tpt = tpt;
+            p2m_tpt = tpt;
         }
     }
-    p2m_tpt = best_tpt;
 }
 
 void Plan::build_tasks()
