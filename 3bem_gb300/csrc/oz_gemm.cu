@@ -273,10 +273,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs a, 
                 my_exp = a.b_exp[(long)a.in_cell[p] * a.nrhs + r];
             }
             const int ea = a.a_exp[(long)ti.x * a.m_pad + row];
-            if (!wait(&accf_bar, tc & 1)) break;
+            // the whole warp goes on or gives up: tcgen05.ld takes all its lanes,
+            // converged
+            if (!__all_sync(0xffffffffu, wait(&accf_bar, tc & 1))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
             for (int c8 = 0; c8 < 32; c8 += 8) {
+                __syncwarp();
                 uint32_t v[OZ_S][8];
                 const uint32_t base = tmem + ((uint32_t)((warp % 4) * 32) << 16) + (warp / 4) * 32 + c8;
 #pragma unroll
@@ -314,9 +317,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs a, 
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (tid == 0 && abort_flag) atomicExch(a.err, 1);
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(OZ_TMEM_COLS));
+    if (tid == 0 && abort_flag) atomicExch(a.err, 1);
 }
 
 unsigned split_grid(long rows) { return (unsigned)std::max<long>(1, std::min<long>((rows + 7) / 8, 152L * 32)); }

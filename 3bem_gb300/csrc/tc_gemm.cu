@@ -307,7 +307,9 @@ __global__ void __launch_bounds__(TC_THREADS_P, 1) tc_gemm_kernel(const TcArgs a
                     drow[cc] = c < ti.w ? a.out_cell[ti.y + c / a.nrhs] * a.nrhs + c % a.nrhs : -1;
                 }
             }
-            if (!wait(&accf_bar[b], bu & 1)) break;
+            // the whole warp goes on or gives up: tcgen05.ld takes all its lanes,
+            // converged
+            if (!__all_sync(0xffffffffu, wait(&accf_bar[b], bu & 1))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = m0 + (warp % 4) * 32 + lane;
 #pragma unroll
@@ -315,6 +317,7 @@ __global__ void __launch_bounds__(TC_THREADS_P, 1) tc_gemm_kernel(const TcArgs a
                 float v[32], w[32];
                 const uint32_t lane_base = tmem + ((uint32_t)((warp % 4) * 32) << 16) + b * 2 * BN + cc * 32;
                 const long my_off = drow[cc] >= 0 ? (long)drow[cc] * a.n : -1;
+                __syncwarp();
                 tmem_ld32(lane_base + BN, v);  // small terms first
                 tmem_ld32(lane_base, w);
 #pragma unroll
@@ -343,9 +346,9 @@ __global__ void __launch_bounds__(TC_THREADS_P, 1) tc_gemm_kernel(const TcArgs a
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (tid == 0 && abort_flag) atomicExch(a.err, 1);
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Sh::TMEM_COLS));
+    if (tid == 0 && abort_flag) atomicExch(a.err, 1);
 }
 
 // v -> three bf16 terms t0 + t1 + t2 (each the rounding of what is left)
