@@ -48,6 +48,9 @@ void check_cusolver(cusolverStatus_t e, const char* what, const char* file, int 
 
 // ------------------------------------------------------------------ helpers
 
+// Bytes of work buffers that the right-hand sides of one pass of an apply may take.
+constexpr double RHS_WORK_BUDGET = 24.0 * (1L << 30);
+
 void TaskSet::add(long target, int count, const double* org,
                   const std::vector<std::pair<long, int>>& srcs, const std::vector<int>& near)
 {
@@ -2172,15 +2175,6 @@ void Plan::build_mixed_ops(Form& F)
         F.tc_c.build(F.Cops.p, n_m2l_ops, F.r_out, F.r_in, stream);
         TBEM_CK(cudaStreamSynchronize(stream));
     }
-    // the FP64 compressed form's M2L from digit planes on the tensor cores
-    // while they (16 bytes per value, twice the operators') stay within 64 GB;
-    // m2l_path 4 keeps the FP64 pipe
-    F.use_oz = F.f64 && opt.m2l_path != 4 && n_m2l_ops > 0 &&
-               16.0 * n_m2l_ops * ((F.r_out + 127) / 128 * 128) * ((F.r_in + 31) / 32 * 32) <= 64e9;
-    if (F.use_oz) {
-        F.oz.build(F.Cops64.p, n_m2l_ops, F.r_out, F.r_in, stream);
-        TBEM_CK(cudaStreamSynchronize(stream));
-    }
     // the auto path keeps the M2L products on the tensor cores when they do
     // not compress (uncompressed 3xBF16 planes)
     const bool auto_tc = opt.m2l_path == 0 && !F.f64 && !F.m2l_compressed && !F.m2l_on_the_fly &&
@@ -2282,6 +2276,32 @@ void Plan::build_mixed_ops(Form& F)
         }
     }
     F.V64.release();
+
+    // The FP64 compressed form's M2L from digit planes on the tensor cores
+    // (m2l_path 4 keeps the FP64 pipe).  The planes take 16 bytes per value
+    // beside the operators' eight, which the transposed apply keeps reading;
+    // they are a choice, so they must not take memory that a later apply of
+    // many right-hand sides or another operator would have had: at most 64 GB,
+    // and half of what the work buffers' budget leaves free (where less than
+    // that budget is free, a sixteenth of it).  Built last, with everything
+    // else of the operator in place.
+    F.use_oz = false;
+    if (F.f64 && opt.m2l_path != 4 && n_m2l_ops > 0) {
+        size_t free_b = 0, total_b = 0;
+        TBEM_CK(cudaMemGetInfo(&free_b, &total_b));
+        const double bytes = 16.0 * n_m2l_ops * ((F.r_out + 127) / 128 * 128) * ((F.r_in + 31) / 32 * 32);
+        const double room = std::max(0.5 * ((double)free_b - RHS_WORK_BUDGET), (double)free_b / 16);
+        if (bytes <= std::min(64e9, room)) {
+            try {
+                F.oz.build(F.Cops64.p, n_m2l_ops, F.r_out, F.r_in, stream);
+                TBEM_CK(cudaStreamSynchronize(stream));
+                F.use_oz = true;
+            } catch (const Error& err) {
+                if (err.code != TBEM_ERR_ALLOC) throw;
+                F.oz = OzPlanes();  // another process took the memory meanwhile: the FP64 pipe
+            }
+        }
+    }
 }
 
 // The compressed precision form.  The bases are those of SVD-compressed M2L
@@ -3368,7 +3388,6 @@ void Plan::apply(const double* x, double* y, int nrhs, cudaStream_t s, bool adj)
 // outputs) within RHS_WORK_BUDGET bytes; at least one.
 int Plan::rhs_chunk(int nrhs) const
 {
-    constexpr double RHS_WORK_BUDGET = 24.0 * (1L << 30);
     const double ncs = (double)stree->cells.size(), nco = (double)otree.cells.size();
     const double N = (double)std::max(n_obs, n_src);
     double per = 8.0 * R * N * 4;  // io copies, strengths, outputs
