@@ -17,10 +17,19 @@
 // as two integers below 2^53, so a tile's result is rounded once, where the
 // FP64 pipe rounds at every addition.
 //
+// What that bounds: an output is off by at most K 2^-58 max|row of A| max|column
+// of B| (K the depth) and a rounding per tile.  The FP64 pipe's bound is
+// relative to sum |a_k b_k|: where a row and a column are graded against each
+// other over more than about 2^11 the digits hold less than it does.  The M2L
+// bases do not grade that way: at rank tolerances 1e-7 to 1e-13 and densities
+// over twelve decades the two paths differ by 1.0e-16 to 4.4e-16 of the
+// result's norm (two operators on the FP64 pipe: 0.5e-16 to 3.2e-16) and, entry
+// by entry, by at most 2.7e-15 of the larger of the entry and the rms (1.3e-15).
+//
 // Why: GB300's FP64 pipe does 1.25 TFLOP/s, and the 494,158 128 x 128 products
-// of a 61,440-point bumpy sphere keep it busy for 13.3 ms; 36 bf16 products of
-// each are 0.6 PFLOP.  That case:
-// M2L 13.3 -> 1.6 ms, the apply 20.0 -> 8.4 ms, its deviation from linearity
+// of a 61,440-point bumpy sphere (16 GFLOP) keep it busy for 13.3 ms; 36 bf16
+// products of each are 0.58 TFLOP, 0.3 ms of the tensor pipe.  That case: M2L
+// 13.3 -> 1.6 ms, the apply 20.0 -> 8.4 ms, its deviation from linearity
 // 9.5e-16 before and 9.7e-16 after.
 //
 // Layout as tc_gemm.cu: persistent, warp-specialized (8 epilogue warps, 4
