@@ -444,8 +444,14 @@ eval_kernel(const EvalArgs<T> a)
 // four to a 4-vector -- serves two targets, and each kernel value is applied
 // to all right-hand sides.  Sums as in eval_kernel (per tile in FP32, folded
 // into a compensated pair; TPT partial sums met by warp shuffles).
-template <int KID, bool TGT_SURF, int TPT, int WIDE>
-__global__ void __launch_bounds__(EVAL_THREADS / 2, 7)
+//
+// SHARED: the compensated pairs sit in shared memory, touched once per tile,
+// and a CTA without second targets skips their pairs.  In registers they leave
+// room for five (double layer) or six CTAs per SM; in shared memory six or seven
+// fit, at 128 shared accesses per thread and tile.  Which one an operator takes:
+// wide_shared (eval_launch.h).
+template <int KID, bool TGT_SURF, int TPT, int WIDE, bool SHARED>
+__global__ void __launch_bounds__(EVAL_THREADS / 2, !SHARED ? 0 : KID == LAP_D && !TGT_SURF ? 6 : 7)
 eval_wide_kernel(const EvalArgs<float> a)
 {
     static_assert(kernel_dim(KID) == 1 && WIDE % 4 == 0, "scalar kernels, packed right-hand sides");
@@ -462,9 +468,7 @@ eval_wide_kernel(const EvalArgs<float> a)
     __shared__ Vec4<float> sl[SPLIT ? EVAL_THREADS : 1];
     __shared__ Vec4<float> snl[DF ? EVAL_THREADS : 1];
     __shared__ Vec4<float> sv[NV][EVAL_THREADS];
-    // the compensated sums, touched once per tile: in registers they left room
-    // for five CTAs per SM (a batch's near field of 64 right-hand sides 8.6 ms)
-    __shared__ float sacc[2][WIDE][NT], slo[2][WIDE][NT];
+    __shared__ float sacc[SHARED ? 2 : 1][SHARED ? WIDE : 1][NT], slo[SHARED ? 2 : 1][SHARED ? WIDE : 1][NT];
 
     const int task = a.item_task[blockIdx.x];
     const int t0 = a.item_start[blockIdx.x];
@@ -505,12 +509,13 @@ eval_wide_kernel(const EvalArgs<float> a)
         }
     }
 
-    float part[2][WIDE];
+    float part[2][WIDE], acc[2][WIDE], lo[2][WIDE];
 #pragma unroll
     for (int q = 0; q < 2; q++)
 #pragma unroll
         for (int i = 0; i < WIDE; i++) {
-            sacc[q][i][threadIdx.x] = slo[q][i][threadIdx.x] = 0.f;
+            if constexpr (SHARED) sacc[q][i][threadIdx.x] = slo[q][i][threadIdx.x] = 0.f;
+            else acc[q][i] = lo[q][i] = 0.f;
             part[q][i] = 0.f;
         }
 
@@ -595,29 +600,34 @@ eval_wide_kernel(const EvalArgs<float> a)
             for (int q = 0; q < NQ; q++)
 #pragma unroll
                 for (int i = 0; i < WIDE; i++) {
-                    float hi = sacc[q][i][threadIdx.x], l = slo[q][i][threadIdx.x];
-                    kahan_add(hi, l, part[q][i]);
-                    sacc[q][i][threadIdx.x] = hi;
-                    slo[q][i][threadIdx.x] = l;
+                    if constexpr (SHARED) {
+                        float hi = sacc[q][i][threadIdx.x], l = slo[q][i][threadIdx.x];
+                        kahan_add(hi, l, part[q][i]);
+                        sacc[q][i][threadIdx.x] = hi;
+                        slo[q][i][threadIdx.x] = l;
+                    } else {
+                        kahan_add(acc[q][i], lo[q][i], part[q][i]);
+                    }
                     part[q][i] = 0.f;
                 }
         };
         // a leaf's last CTA often holds no second targets at all
-        if (t0 + HALF < ntgt) {
+        if (!SHARED || t0 + HALF < ntgt) {
             if (act[0] || act[1]) pairs(std::integral_constant<int, 2>());
-        } else if (act[0]) {
-            pairs(std::integral_constant<int, 1>());
+        } else if constexpr (SHARED) {
+            if (act[0]) pairs(std::integral_constant<int, 1>());
         }
         __syncthreads();
     }
-    float acc[2][WIDE], lo[2][WIDE];
+    if constexpr (SHARED) {
 #pragma unroll
-    for (int q = 0; q < 2; q++)
+        for (int q = 0; q < 2; q++)
 #pragma unroll
-        for (int i = 0; i < WIDE; i++) {
-            acc[q][i] = sacc[q][i][threadIdx.x];
-            lo[q][i] = slo[q][i][threadIdx.x];
-        }
+            for (int i = 0; i < WIDE; i++) {
+                acc[q][i] = sacc[q][i][threadIdx.x];
+                lo[q][i] = slo[q][i][threadIdx.x];
+            }
+    }
     // the TPT partial sums of a target pair (consecutive lanes of one warp)
 #pragma unroll
     for (int off = TPT / 2; off > 0; off /= 2) {

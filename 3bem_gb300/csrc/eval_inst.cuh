@@ -7,7 +7,7 @@ namespace tbem {
 
 namespace {
 template <typename T, bool TR, bool TS, bool SS, int TPT>
-void go_tpt(int nr, int n_items, const EvalArgs<T>& a, cudaStream_t s)
+void go_tpt(const EvalLaunch& L, int nr, int n_items, const EvalArgs<T>& a, cudaStream_t s)
 {
     if (nr == 1) {
         eval_kernel<EVAL_KID, TR, T, 1, TS, SS, TPT><<<n_items, EVAL_THREADS, 0, s>>>(a);
@@ -16,7 +16,9 @@ void go_tpt(int nr, int n_items, const EvalArgs<T>& a, cudaStream_t s)
     if constexpr (sizeof(T) == 4 && kernel_dim(EVAL_KID) == 1 && kernel_space_dim(EVAL_KID) == 3 &&
                   !TR && !SS && TPT != EVAL_PER_ITEM) {
         if (nr == EVAL_NR_WIDE) {
-            eval_wide_kernel<EVAL_KID, TS, TPT, EVAL_NR_WIDE><<<n_items, EVAL_THREADS / 2, 0, s>>>(a);
+            auto kern = L.wide_shared ? eval_wide_kernel<EVAL_KID, TS, TPT, EVAL_NR_WIDE, true>
+                                      : eval_wide_kernel<EVAL_KID, TS, TPT, EVAL_NR_WIDE, false>;
+            kern<<<n_items, EVAL_THREADS / 2, 0, s>>>(a);
             return;
         }
     }
@@ -24,8 +26,9 @@ void go_tpt(int nr, int n_items, const EvalArgs<T>& a, cudaStream_t s)
 }
 
 template <typename T, bool TR, bool TS, bool SS>
-cudaError_t go(int nr, int n_items, int tpt, const void* args, cudaStream_t s)
+cudaError_t go(const EvalLaunch& L, int nr, int tpt, const void* args, cudaStream_t s)
 {
+    const int n_items = L.n_items;
     const EvalArgs<T>& a = *static_cast<const EvalArgs<T>*>(args);
     if (n_items <= 0) return cudaSuccess;
     // the FP64 point-to-point passes take it per item (their pace is the FP64
@@ -33,18 +36,18 @@ cudaError_t go(int nr, int n_items, int tpt, const void* args, cudaStream_t s)
     // and the points-to-check-surface pass (1, 2, 4) have autotuned variants;
     // every other pass uses 4
     if constexpr (sizeof(T) == 8 && !TS && !SS) {
-        if (tpt == EVAL_PER_ITEM) go_tpt<T, TR, TS, SS, EVAL_PER_ITEM>(nr, n_items, a, s);
+        if (tpt == EVAL_PER_ITEM) go_tpt<T, TR, TS, SS, EVAL_PER_ITEM>(L, nr, n_items, a, s);
         else return cudaErrorInvalidValue;
     } else if constexpr (!TR && !TS && !SS) {
-        if (tpt == 2) go_tpt<T, TR, TS, SS, 2>(nr, n_items, a, s);
-        else if (tpt == 8) go_tpt<T, TR, TS, SS, 8>(nr, n_items, a, s);
-        else go_tpt<T, TR, TS, SS, 4>(nr, n_items, a, s);
+        if (tpt == 2) go_tpt<T, TR, TS, SS, 2>(L, nr, n_items, a, s);
+        else if (tpt == 8) go_tpt<T, TR, TS, SS, 8>(L, nr, n_items, a, s);
+        else go_tpt<T, TR, TS, SS, 4>(L, nr, n_items, a, s);
     } else if constexpr (!TR && TS && !SS) {
-        if (tpt == 1) go_tpt<T, TR, TS, SS, 1>(nr, n_items, a, s);
-        else if (tpt == 2) go_tpt<T, TR, TS, SS, 2>(nr, n_items, a, s);
-        else go_tpt<T, TR, TS, SS, 4>(nr, n_items, a, s);
+        if (tpt == 1) go_tpt<T, TR, TS, SS, 1>(L, nr, n_items, a, s);
+        else if (tpt == 2) go_tpt<T, TR, TS, SS, 2>(L, nr, n_items, a, s);
+        else go_tpt<T, TR, TS, SS, 4>(L, nr, n_items, a, s);
     } else {
-        go_tpt<T, TR, TS, SS, 4>(nr, n_items, a, s);
+        go_tpt<T, TR, TS, SS, 4>(L, nr, n_items, a, s);
     }
     return cudaGetLastError();
 }
@@ -56,14 +59,14 @@ cudaError_t go_t(const EvalLaunch& L, const void* args, cudaStream_t s)
     const int nr = eval_rhs_block(L, sizeof(T) == 4, a.nrhs - a.rhs0);
     const int idx = (L.trans ? 4 : 0) + (L.tgt_surf ? 2 : 0) + (L.src_surf ? 1 : 0);
     switch (idx) {
-    case 0: return go<T, false, false, false>(nr, L.n_items, L.tpt, args, s);
-    case 1: return go<T, false, false, true>(nr, L.n_items, 4, args, s);
-    case 2: return go<T, false, true, false>(nr, L.n_items, L.tpt, args, s);
-    case 3: return go<T, false, true, true>(nr, L.n_items, 4, args, s);
-    case 4: return go<T, true, false, false>(nr, L.n_items, L.tpt, args, s);
-    case 5: return go<T, true, false, true>(nr, L.n_items, 4, args, s);
-    case 6: return go<T, true, true, false>(nr, L.n_items, 4, args, s);
-    default: return go<T, true, true, true>(nr, L.n_items, 4, args, s);
+    case 0: return go<T, false, false, false>(L, nr, L.tpt, args, s);
+    case 1: return go<T, false, false, true>(L, nr, 4, args, s);
+    case 2: return go<T, false, true, false>(L, nr, L.tpt, args, s);
+    case 3: return go<T, false, true, true>(L, nr, 4, args, s);
+    case 4: return go<T, true, false, false>(L, nr, L.tpt, args, s);
+    case 5: return go<T, true, false, true>(L, nr, 4, args, s);
+    case 6: return go<T, true, true, false>(L, nr, 4, args, s);
+    default: return go<T, true, true, true>(L, nr, 4, args, s);
     }
 }
 }  // namespace

@@ -13,6 +13,7 @@ struct EvalLaunch {
     int n_items;
     int tpt = 4;  // threads per target (point-to-point: EVAL_PER_ITEM in FP64, 2, 4 or 8 in FP32;
                   // 1, 2 or 4 for points to a check surface; 4 otherwise)
+    bool wide_shared = false;  // many right-hand sides: the sums in shared memory
 };
 
 // One function per kernel id (eval_k<id>.cu) so that the instantiations
@@ -49,6 +50,23 @@ inline int eval_rhs_block(const EvalLaunch& L, bool fp32, int remaining)
         remaining >= EVAL_NR_WIDE)
         return EVAL_NR_WIDE;
     return EVAL_NR;
+}
+
+// Whether an operator's passes of many right-hand sides (both of them) keep
+// their sums in shared memory, from the CTAs of its point-to-point pass and
+// that pass's threads per target.  What it buys is occupancy, so small batches
+// lose: with fewer CTAs than fit anyway the shared accesses only cost, and with
+// eight threads per target a thread has 16 pairs per tile to set against them,
+// of which the single layer's are a third of the double layer's work.  Batches
+// of 3 to 16 spheres, 16 to 64 right-hand sides (registers / shared, us; CTAs
+// per SM): double layer 972 / 1125 (2.6), 1277 / 1283 (4.4), 1320 / 1258 (4.8),
+// 1826 / 1603 (6.6), 12204 / 10799 (26); single layer with eight threads 662 /
+// 749 (2.6), 922 / 942 (6.6), 2042 / 2281 (9.7), with four 1365 / 1412 (7.5),
+// 1903 / 1686 (9.7), 3332 / 3603 (10.2), 4824 / 4644 (15), 7661 / 7505 (26).
+inline bool wide_shared(int kid, int p2p_items, int p2p_tpt)
+{
+    if (kid == LAP_D) return p2p_items >= 700;
+    return p2p_tpt <= 4 && p2p_items >= 9 * 152;
 }
 
 // Threads per target of the direct sum: a warp until 32 targets per CTA give

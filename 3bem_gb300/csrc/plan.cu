@@ -2910,6 +2910,10 @@ void Plan::eval(const TaskSet& ts, int ekid, bool tgt_surf, bool src_surf, const
     const TaskSet::Items& it = cut->second;
     TaskSet::fill_items(a, it);
     EvalLaunch Lc{ekid, trans, tgt_surf, src_surf, it.n, it.tpt};
+    if (sizeof(T) == 4 && nrhs >= EVAL_NR_WIDE) {
+        auto near = p2p.cuts.find(p2p_tpt);
+        Lc.wide_shared = near != p2p.cuts.end() && wide_shared(kid, near->second.n, p2p_tpt);
+    }
     for (int r0 = 0; r0 < nrhs;) {
         a.rhs0 = r0;
         TBEM_CK(launch_eval<T>(Lc, a, s));
