@@ -233,7 +233,7 @@ double fma_peak(int device)
 
 struct TbemCsr {
     long n_rows = 0, n_cols = 0, nnz = 0;
-    int lanes = 32;  // lanes per row of the SpMV kernel
+    int lanes = 32;  // lanes per row of the SpMV kernel (csr_lanes, csr_block_lanes)
     tbem::DBuf<long> rowptr;
     tbem::DBuf<int> col;        // n_cols <= 2^31 - 1
     tbem::DBuf<long> col_wide;  // else
@@ -242,36 +242,75 @@ struct TbemCsr {
 
 namespace {
 // y (+)= A x on stream s (A non-empty)
-void csr_launch(const TbemCsr* A, const double* x, double* y, int nrhs, int add, cudaStream_t s)
+int device_sms()
 {
-    const int L = A->lanes;
     int dev = 0, sms = 0;
     TBEM_CK(cudaGetDevice(&dev));
     TBEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const long need = (A->n_rows * L + CSR_THREADS - 1) / CSR_THREADS;
-    const unsigned blocks = (unsigned)std::min<long>(need, (long)CSR_CTAS_PER_SM * std::max(sms, 1));
-    auto with_lanes = [&](auto lanes, const auto* col) {
+    return std::max(sms, 1);
+}
+
+// Lanes per row: the fewest that take a mean row in one unrolled step (its
+// latency), but no more than give the chip a thousand threads per SM: from
+// there on fewer lanes add less on the FP64 pipe.  The rows of a warp walk in
+// step with the longest of them, so the matrix's longest row also sets a
+// least: 24 steps, or twice the steps of an even share where that is more
+// (100,000 rows, one of a thousand with 5,000 entries and 12 else: 178 us with
+// 4 lanes, 99 with 16; one row of 200,000 among rows of 20: 4.8 ms with 4, 0.67
+// with 32; one of a hundred with 500 entries and 50 else: 62 with 4, 56 with 8).
+int csr_lanes(const long* row_ptrs, long n_rows, long nnz, int sms)
+{
+    const double mean = n_rows > 0 ? (double)nnz / (double)n_rows : 0.0;
+    const long threads = 1024L * sms;
+    long longest = 0;
+    for (long i = 0; i < n_rows; i++) longest = std::max(longest, row_ptrs[i + 1] - row_ptrs[i]);
+    const long most = CSR_UNROLL * std::max(24L, nnz / (2 * threads));  // entries per lane
+    int lanes = mean <= 4 * CSR_UNROLL ? 4 : mean <= 8 * CSR_UNROLL ? 8 : mean <= 16 * CSR_UNROLL ? 16 : 32;
+    while (lanes > 4 && n_rows * (lanes / 2) >= threads) lanes /= 2;
+    while (lanes < 32 && longest > most * lanes) lanes *= 2;
+    return lanes;
+}
+
+// The lanes of a launch of `nr` right-hand sides: long mean rows read best in
+// longer pieces where the gathers do not pace (40,000 rows of 500, 1,000 and
+// 2,000 entries, 4 / 16 lanes, us: one right-hand side 97 / 79, 163 / 122, 296
+// / 207; two 117 / 127, 200 / 212, 364 / 382; four 193 / 218, 351 / 324, 666 /
+// 591).
+int csr_block_lanes(const TbemCsr* A, int nr)
+{
+    const double mean = (double)A->nnz / (double)A->n_rows;
+    const bool pieces = (nr == 1 && mean > 256) || (nr == CSR_RHS && mean > 768);
+    return pieces ? std::max(A->lanes, 16) : A->lanes;
+}
+
+void csr_launch(const TbemCsr* A, const double* x, double* y, int nrhs, int add, cudaStream_t s)
+{
+    const int sms = device_sms();
+    auto block = [&](auto lanes, const auto* col, int r0, int nr) {
         constexpr int LL = decltype(lanes)::value;
-        for (int r0 = 0; r0 < nrhs; r0 += CSR_RHS) {
-            const double* xr = x + (long)r0 * A->n_cols;
-            double* yr = y + (long)r0 * A->n_rows;
-            auto launch = [&](auto kern) {
-                kern<<<blocks, CSR_THREADS, 0, s>>>(A->rowptr.p, col, A->val.p, xr, yr, A->n_rows, A->n_cols, add);
-            };
-            using I = std::remove_const_t<std::remove_pointer_t<decltype(col)>>;
-            switch (std::min(nrhs - r0, CSR_RHS)) {
-            case 1: launch(csr_kernel<LL, 1, I>); break;
-            case 2: launch(csr_kernel<LL, 2, I>); break;
-            case 3: launch(csr_kernel<LL, 3, I>); break;
-            default: launch(csr_kernel<LL, 4, I>);
-            }
+        const long need = (A->n_rows * LL + CSR_THREADS - 1) / CSR_THREADS;
+        const unsigned blocks = (unsigned)std::min<long>(need, (long)CSR_CTAS_PER_SM * sms);
+        const double* xr = x + (long)r0 * A->n_cols;
+        double* yr = y + (long)r0 * A->n_rows;
+        auto launch = [&](auto kern) {
+            kern<<<blocks, CSR_THREADS, 0, s>>>(A->rowptr.p, col, A->val.p, xr, yr, A->n_rows, A->n_cols, add);
+        };
+        using I = std::remove_const_t<std::remove_pointer_t<decltype(col)>>;
+        switch (nr) {
+        case 1: launch(csr_kernel<LL, 1, I>); break;
+        case 2: launch(csr_kernel<LL, 2, I>); break;
+        case 3: launch(csr_kernel<LL, 3, I>); break;
+        default: launch(csr_kernel<LL, 4, I>);
         }
     };
     auto go = [&](const auto* col) {
-        if (L == 4) with_lanes(std::integral_constant<int, 4>(), col);
-        else if (L == 8) with_lanes(std::integral_constant<int, 8>(), col);
-        else if (L == 16) with_lanes(std::integral_constant<int, 16>(), col);
-        else with_lanes(std::integral_constant<int, 32>(), col);
+        for (int r0 = 0; r0 < nrhs; r0 += CSR_RHS) {
+            const int nr = std::min(nrhs - r0, CSR_RHS), L = csr_block_lanes(A, nr);
+            if (L == 4) block(std::integral_constant<int, 4>(), col, r0, nr);
+            else if (L == 8) block(std::integral_constant<int, 8>(), col, r0, nr);
+            else if (L == 16) block(std::integral_constant<int, 16>(), col, r0, nr);
+            else block(std::integral_constant<int, 32>(), col, r0, nr);
+        }
     };
     if (A->col.p) go(A->col.p);
     else go(A->col_wide.p);
@@ -391,12 +430,7 @@ int tbem_csr_create(long n_rows, long n_cols, const double* values, const long* 
         h->n_rows = n_rows;
         h->n_cols = n_cols;
         h->nnz = nnz;
-        // lanes per row: the fewest that take a mean row in one unrolled step
-        // (its latency), but no more than give the chip a thousand threads
-        // per SM: from there on fewer lanes add less on the FP64 pipe
-        const double mean = n_rows > 0 ? (double)nnz / (double)n_rows : 0.0;
-        h->lanes = mean <= 4 * CSR_UNROLL ? 4 : mean <= 8 * CSR_UNROLL ? 8 : mean <= 16 * CSR_UNROLL ? 16 : 32;
-        while (h->lanes > 4 && n_rows * (h->lanes / 2) >= 152L * 1024) h->lanes /= 2;
+        h->lanes = csr_lanes(row_ptrs, n_rows, nnz, device_sms());
         h->rowptr.upload(row_ptrs, (size_t)n_rows + 1);
         if (nnz > 0) {
             if (wide) h->col_wide.upload(column_indices, (size_t)nnz);
