@@ -69,10 +69,44 @@ inline bool wide_shared(int kid, int p2p_items, int p2p_tpt)
     return p2p_tpt <= 4 && p2p_items >= 9 * 152;
 }
 
-// Threads per target of the direct sum: a warp until 32 targets per CTA give
-// every SM eight CTAs (with four threads per target, 6,144 points were 192 CTAs
-// on 152 SMs: traction 5.0 ms, 3.5 with a warp).
-inline int direct_tpt(long n_obs) { return n_obs < 152L * 8 * (EVAL_THREADS / 4) ? 32 : 4; }
+// SMs of the current device (152 where there is none to ask: argument checks
+// come before any launch).
+inline int sm_count()
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
+        return sms;
+    cudaGetLastError();
+    return 152;
+}
+
+// Threads per target of the direct sum, 8, 16 or 32, one number for all its
+// CTAs of EVAL_THREADS / tpt targets.  Every target sees all sources, so the
+// pass lasts as long as the SM with most targets, ceil(CTAs / SMs) * targets
+// per CTA, times what staging the sources adds per pair: a CTA stages each
+// source once for its targets, about 1/512 of the pair work per thread per
+// target.  Few points need many threads for an even share, where shares are
+// even anyway fewer threads stage less.  Measured (4 / 8 / 16 / 32 threads,
+// us): single layer, 4,705 points 886 / 867 / 879 / 897, 4,900 points 1449 /
+// 1174 / 1044 / 1005, 12,000 points 4480 / 3831 / 3886 / 4013; traction, 3,457
+// points 1545 / 1541 / 1247 / 1279, 6,145 points 4656 / 3601 / 3635 / 3440.  Over
+// 46 sizes, kernels and counts of right-hand sides the rule's choice is within
+// 4 % of the best.
+inline int direct_tpt(long n_obs, int sms)
+{
+    int best = 8;
+    double least = 1e300;
+    for (int tpt : {8, 16, 32}) {
+        const long targets = EVAL_THREADS / tpt, ctas = (n_obs + targets - 1) / targets;
+        const double cost = (double)((ctas + sms - 1) / sms * targets) * (1.0 + tpt / 512.0);
+        if (cost < least) {
+            least = cost;
+            best = tpt;
+        }
+    }
+    return best;
+}
 
 template <typename T>
 inline cudaError_t launch_eval(const EvalLaunch& L, const EvalArgs<T>& a, cudaStream_t s)

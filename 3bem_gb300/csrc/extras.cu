@@ -242,14 +242,6 @@ struct TbemCsr {
 
 namespace {
 // y (+)= A x on stream s (A non-empty)
-int device_sms()
-{
-    int dev = 0, sms = 0;
-    TBEM_CK(cudaGetDevice(&dev));
-    TBEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    return std::max(sms, 1);
-}
-
 // Lanes per row: the fewest that take a mean row in one unrolled step (its
 // latency), but no more than give the chip a thousand threads per SM: from
 // there on fewer lanes add less on the FP64 pipe.  The rows of a warp walk in
@@ -285,7 +277,7 @@ int csr_block_lanes(const TbemCsr* A, int nr)
 
 void csr_launch(const TbemCsr* A, const double* x, double* y, int nrhs, int add, cudaStream_t s)
 {
-    const int sms = device_sms();
+    const int sms = tbem::sm_count();
     auto block = [&](auto lanes, const auto* col, int r0, int nr) {
         constexpr int LL = decltype(lanes)::value;
         const long need = (A->n_rows * LL + CSR_THREADS - 1) / CSR_THREADS;
@@ -366,8 +358,8 @@ int tbem_direct_apply(int kernel, const double* kernel_params, const double* obs
             double org[3] = {0, 0, 0};
             for (long b = 0; b < n_obs; b += chunk)
                 ts.add(b, (int)std::min<long>(chunk, n_obs - b), org, {{0L, (int)n_src}});
-            const int cut = TaskSet::SPLIT + direct_tpt(n_obs);
-            ts.upload({cut});
+            const int tpt = direct_tpt(n_obs, sm_count());
+            ts.upload({tpt});
             EvalArgs<double> a{};
             ts.fill(a);
             a.t_xyz = ol.p;
@@ -382,9 +374,10 @@ int tbem_direct_apply(int kernel, const double* kernel_params, const double* obs
             a.add = 0;
             a.c2 = kp.c2;
             a.scale = kp.scale;
-            const TaskSet::Items& it = ts.cuts.at(cut);
-            TaskSet::fill_items(a, it);
-            EvalLaunch L{kernel, false, false, false, it.n, it.tpt};
+            const TaskSet::Items& it = ts.cuts.at(tpt);
+            TaskSet::fill_items(a, it);  // one number of threads per target for all items
+            for (a.tpt_log = 0; (1 << a.tpt_log) < tpt;) a.tpt_log++;
+            EvalLaunch L{kernel, false, false, false, it.n, EVAL_PER_ITEM};
             for (int r0 = 0; r0 < n_rhs; r0 += (n_rhs - r0 > 1 ? EVAL_NR : 1)) {
                 a.rhs0 = r0;
                 TBEM_CK(launch_eval<double>(L, a, s));
@@ -430,7 +423,7 @@ int tbem_csr_create(long n_rows, long n_cols, const double* values, const long* 
         h->n_rows = n_rows;
         h->n_cols = n_cols;
         h->nnz = nnz;
-        h->lanes = csr_lanes(row_ptrs, n_rows, nnz, device_sms());
+        h->lanes = csr_lanes(row_ptrs, n_rows, nnz, sm_count());
         h->rowptr.upload(row_ptrs, (size_t)n_rows + 1);
         if (nnz > 0) {
             if (wide) h->col_wide.upload(column_indices, (size_t)nnz);

@@ -145,10 +145,20 @@ extern "C" int tbem_direct_apply_noalloc(int kernel, const double* kernel_params
                                           " doubles");
         const long n_tasks = (n_obs + NOALLOC_CHUNK - 1) / NOALLOC_CHUNK;
         const long last = n_obs - (n_tasks - 1) * NOALLOC_CHUNK;
-        const int tpt = direct_tpt(n_obs), tpb = EVAL_THREADS / tpt;
-        const long n_items = (n_tasks - 1) * (NOALLOC_CHUNK / tpb) + (last + tpb - 1) / tpb;
-        const TaskLayout TL = layout((int)std::min<long>(n_tasks, INT32_MAX),
-                                     (int)std::min<long>(n_items, INT32_MAX));
+        // threads per target as the direct sum's, fewer where their work items
+        // would not fit the scratch (from four on it is the entry's limit)
+        int tpt = direct_tpt(n_obs, sm_count());
+        auto items_of = [&](int threads) {
+            const long targets = EVAL_THREADS / threads;
+            return (n_tasks - 1) * (NOALLOC_CHUNK / targets) + (last + targets - 1) / targets;
+        };
+        auto layout_of = [&](int threads) {
+            return layout((int)std::min<long>(n_tasks, INT32_MAX), (int)std::min<long>(items_of(threads), INT32_MAX));
+        };
+        while (tpt > 4 && (items_of(tpt) > INT32_MAX || layout_of(tpt).total > NOALLOC_TASK_BYTES)) tpt /= 2;
+        const int tpb = EVAL_THREADS / tpt;
+        const long n_items = items_of(tpt);
+        const TaskLayout TL = layout_of(tpt);
         if (n_items > INT32_MAX || TL.total > NOALLOC_TASK_BYTES)
             throw Error(TBEM_ERR_ARG, "tbem_direct_apply_noalloc: n_obs = " + std::to_string(n_obs) +
                                           " needs more work-item descriptors than the scratch "
@@ -179,7 +189,7 @@ extern "C" int tbem_direct_apply_noalloc(int kernel, const double* kernel_params
         a.item_task = reinterpret_cast<const int*>(base + TL.item_task);
         a.item_start = reinterpret_cast<const int*>(base + TL.item_start);
         a.item_tpt = nullptr;
-        a.tpt_log = tpt == 32 ? 5 : 2;
+        for (a.tpt_log = 0; (1 << a.tpt_log) < tpt;) a.tpt_log++;
         a.task_tgt = reinterpret_cast<const long*>(base + TL.task_tgt);
         a.task_tgt_count = reinterpret_cast<const int*>(base + TL.task_count);
         a.task_origin = reinterpret_cast<const double*>(base + TL.task_origin);
