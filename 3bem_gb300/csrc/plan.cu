@@ -1269,38 +1269,63 @@ void Plan::autotune_tc()
 
 namespace {
 // A timed variant replaces the best one so far only when it is faster by more
-// than repeated timings differ (0.3 % for the FP32 passes, up to 3 % for the
-// FP64 ones, over four constructions of 40 operators): variants that tie would
-// otherwise fall either way from one construction to the next, and with them
-// the summation order, which shows in the results (points to check surfaces in
-// the plain form: its pseudo-inverses turn it into 1e-8; the FP32 near field:
-// 3e-7).
-constexpr float AUTOTUNE_MARGIN_FP32 = 0.99f, AUTOTUNE_MARGIN_FP64 = 0.97f;
+// than repeated timings differ (half a percent for the FP32 passes, up to 4 %
+// between two of the FP64 ones, over six constructions of 40 operators):
+// variants that tie would otherwise fall either way from one construction to
+// the next, and with them the summation order, which shows in the results
+// (points to check surfaces in the plain form: its pseudo-inverses turn it into
+// 1e-8; the FP32 near field: 3e-7).  In the FP64 near field it does not (1e-15).
+constexpr float AUTOTUNE_MARGIN_FP32 = 0.99f, AUTOTUNE_MARGIN_FP64 = 0.96f;
 
-// Time of one launch of `run` on `s`, in ms.  Passes of small operators last
-// 6 to 50 us, of which an event pair resolves half a percent, and a lone
-// launch's own jitter is several: each sample is a row of launches of
-// AUTOTUNE_SPAN ms in all, and the fastest of four samples counts.  Launches
-// of 20 ms and more repeat within the margin and are timed twice.
-constexpr float AUTOTUNE_SPAN = 0.3f;
+// The fastest of `variants` (threads per target; run(v) launches one): each is
+// timed shortly, and, where the choice shows (margin below 1), those within 8 %
+// of the fastest again and longer: there the first in order stays unless
+// another is faster by the margin.  Passes of
+// small operators last 6 to 50 us, of which an event pair resolves half a
+// percent, and a lone launch's own jitter is several: a sample is a row of
+// launches of `span` ms in all, and the fastest sample counts.  (Rows of 0.1 ms
+// spread three times as much as rows of 0.2 to 0.3 ms.)
 template <typename F>
-float time_launch(cudaEvent_t e0, cudaEvent_t e1, cudaStream_t s, F&& run)
+int fastest_variant(const std::vector<int>& variants, float margin, cudaStream_t s, F&& run)
 {
-    auto row = [&](int n) {
-        TBEM_CK(cudaEventRecord(e0, s));
-        for (int i = 0; i < n; i++) run();
-        TBEM_CK(cudaEventRecord(e1, s));
-        TBEM_CK(cudaEventSynchronize(e1));
+    ScopedEvent e0, e1;
+    auto row = [&](int v, int n) {
+        TBEM_CK(cudaEventRecord(e0.e, s));
+        for (int i = 0; i < n; i++) run(v);
+        TBEM_CK(cudaEventRecord(e1.e, s));
+        TBEM_CK(cudaEventSynchronize(e1.e));
         float t = 0.f;
-        TBEM_CK(cudaEventElapsedTime(&t, e0, e1));
+        TBEM_CK(cudaEventElapsedTime(&t, e0.e, e1.e));
         return t / n;
     };
-    row(1);  // warms the caches
-    float best = row(1);
-    const int n = (int)std::min(32.f, std::max(1.f, std::ceil(AUTOTUNE_SPAN / std::max(best, 1e-3f))));
-    if (n > 1) best = 1e30f;  // a lone launch is no sample of a row
-    for (int rep = 0; rep < (best > 20.f && n == 1 ? 1 : 4); rep++) best = std::min(best, row(n));
-    return best;
+    auto rows = [&](int v, float ms, float span, int samples) {
+        const int n = (int)std::min(48.f, std::max(1.f, std::ceil(span / std::max(ms, 1e-3f))));
+        float best = 1e30f;
+        for (int i = 0; i < samples; i++) best = std::min(best, row(v, n));
+        return best;
+    };
+    std::vector<float> ms(variants.size());
+    float least = 1e30f;
+    for (size_t i = 0; i < variants.size(); i++) {
+        row(variants[i], 1);  // warms the caches
+        ms[i] = row(variants[i], 1);
+        if (ms[i] < 20.f) ms[i] = rows(variants[i], ms[i], 0.05f, 2);  // (longer launches repeat)
+        least = std::min(least, ms[i]);
+    }
+    std::vector<size_t> close;
+    for (size_t i = 0; i < variants.size(); i++)
+        if (ms[i] <= (margin < 1.f ? 1.08f : 1.f) * least) close.push_back(i);
+    int pick = variants[close[0]];
+    float best = 1e30f;
+    if (close.size() > 1)
+        for (size_t i : close) {
+            const float t = ms[i] < 20.f ? rows(variants[i], ms[i], 0.2f, 3) : ms[i];
+            if (t < margin * best) {
+                best = t;
+                pick = variants[i];
+            }
+        }
+    return pick;
 }
 }  // namespace
 
@@ -1314,22 +1339,14 @@ void Plan::autotune_p2p()
     const bool mixed = f.mixed && !f.f64;  // FP32 evaluation passes
     if (mixed) TBEM_CK(cudaMemsetAsync(s32.p, 0, sizeof(float) * R * n_src, stream));
     else TBEM_CK(cudaMemsetAsync(s64.p, 0, sizeof(double) * R * n_src, stream));
-    ScopedEvent t0, t1;
-    float best = 1e30f;
-    for (int tpt : {4, 2, 8}) {
-        const float ms = time_launch(t0.e, t1.e, stream, [&] {
-            if (mixed)
-                eval<float>(p2p, kid, false, false, otree, dobs, 0, *dsrc, 0, s32.p, n_src,
-                            nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, tpt);
-            else
-                eval<double>(p2p, kid, false, false, otree, dobs, 0, *dsrc, 0, s64.p, n_src,
-                             nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, tpt);
-        });
-        if (ms < (mixed ? AUTOTUNE_MARGIN_FP32 : AUTOTUNE_MARGIN_FP64) * best) {
-            best = ms;
-            p2p_tpt = tpt;
-        }
-    }
+    p2p_tpt = fastest_variant({4, 2, 8}, mixed ? AUTOTUNE_MARGIN_FP32 : 1.f, stream, [&](int tpt) {
+        if (mixed)
+            eval<float>(p2p, kid, false, false, otree, dobs, 0, *dsrc, 0, s32.p, n_src,
+                        nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, tpt);
+        else
+            eval<double>(p2p, kid, false, false, otree, dobs, 0, *dsrc, 0, s64.p, n_src,
+                         nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, tpt);
+    });
 }
 
 // Picks the points-to-check-surface pass's threads per target (1, 2 or 4)
@@ -1341,22 +1358,14 @@ void Plan::autotune_p2m()
     const bool mixed = f.mixed && !f.f64;  // FP32 evaluation passes
     if (mixed) TBEM_CK(cudaMemsetAsync(s32.p, 0, sizeof(float) * R * n_src, stream));
     else TBEM_CK(cudaMemsetAsync(s64.p, 0, sizeof(double) * R * n_src, stream));
-    ScopedEvent t0, t1;
-    float best = 1e30f;
-    for (int tpt : {4, 2, 1}) {
-        const float ms = time_launch(t0.e, t1.e, stream, [&] {
-            if (mixed)
-                eval<float>(p2m, f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s32.p, n_src,
-                            nullptr, nullptr, 0, cu32.p, 0, 1, stream, false, tpt);
-            else
-                eval<double>(p2m, f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s64.p, n_src,
-                             nullptr, nullptr, 0, cu64.p, 0, 1, stream, false, tpt);
-        });
-        if (ms < (mixed ? AUTOTUNE_MARGIN_FP32 : AUTOTUNE_MARGIN_FP64) * best) {
-            best = ms;
-            p2m_tpt = tpt;
-        }
-    }
+    p2m_tpt = fastest_variant({4, 2, 1}, mixed ? AUTOTUNE_MARGIN_FP32 : AUTOTUNE_MARGIN_FP64, stream, [&](int tpt) {
+        if (mixed)
+            eval<float>(p2m, f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s32.p, n_src,
+                        nullptr, nullptr, 0, cu32.p, 0, 1, stream, false, tpt);
+        else
+            eval<double>(p2m, f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s64.p, n_src,
+                         nullptr, nullptr, 0, cu64.p, 0, 1, stream, false, tpt);
+    });
 }
 
 void Plan::build_tasks()
