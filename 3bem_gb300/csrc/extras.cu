@@ -68,6 +68,12 @@ __global__ void weight_kernel(const double* x, const double* w, double* s, long 
         s[t] = w[t % N] * x[t];
 }
 
+__global__ void narrow_kernel(const long* in, int* out, long n)
+{
+    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
+        out[t] = (int)in[t];
+}
+
 // y = A x (add = 0) or y += A x (add = 1).  L lanes per row (L chosen per
 // matrix from its mean row length): a lane takes the row's entries k = b +
 // lane, + L, ..., CSR_UNROLL of them per step, and the L partial sums meet in
@@ -403,18 +409,14 @@ int tbem_csr_create(long n_rows, long n_cols, const double* values, const long* 
             if (row_ptrs[i + 1] < row_ptrs[i]) throw Error(TBEM_ERR_ARG, "row_ptrs must not decrease");
         const long nnz = row_ptrs[n_rows];
         if (nnz > 0 && (!values || !column_indices)) throw Error(TBEM_ERR_ARG, "null values");
-        // column check (and narrowing) on all host cores, in blocks (one flag per block)
-        const bool wide = n_cols > (long)INT32_MAX;
-        std::vector<int> narrow(wide ? 0 : nnz);
+        // column check on all host cores, in blocks (one flag per block)
         const long block = 1 << 20, n_blocks = (nnz + block - 1) / block;
         std::vector<char> bad(n_blocks, 0);
         nf::parallel_for(
             n_blocks,
             [&](long b) {
-                for (long k = b * block; k < std::min(nnz, (b + 1) * block); k++) {
+                for (long k = b * block; k < std::min(nnz, (b + 1) * block); k++)
                     if (column_indices[k] < 0 || column_indices[k] >= n_cols) bad[b] = 1;
-                    if (!wide) narrow[k] = (int)column_indices[k];
-                }
             },
             1);
         if (std::find(bad.begin(), bad.end(), 1) != bad.end())
@@ -426,9 +428,18 @@ int tbem_csr_create(long n_rows, long n_cols, const double* values, const long* 
         h->lanes = csr_lanes(row_ptrs, n_rows, nnz, sm_count());
         h->rowptr.upload(row_ptrs, (size_t)n_rows + 1);
         if (nnz > 0) {
-            if (wide) h->col_wide.upload(column_indices, (size_t)nnz);
-            else h->col.upload(narrow);
-            h->val.upload(values, (size_t)nnz);
+            // narrowed on the device (on the host its fresh pages took longer
+            // than the copy: 9.2 M entries 4.65 ms, 2.3 without)
+            DBuf<long> full;
+            full.upload(column_indices, (size_t)nnz);
+            if (n_cols > (long)INT32_MAX) {
+                h->col_wide = std::move(full);
+            } else {
+                h->col.alloc((size_t)nnz);
+                narrow_kernel<<<(unsigned)std::min<long>((nnz + 255) / 256, 9728), 256>>>(full.p, h->col.p, nnz);
+                TBEM_CK(cudaGetLastError());
+            }
+            h->val.upload(values, (size_t)nnz);  // (waits for the narrowing as well)
         }
         *out = h.release();
         return TBEM_OK;
