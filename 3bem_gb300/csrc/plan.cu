@@ -1269,22 +1269,23 @@ void Plan::autotune_tc()
 
 namespace {
 // A timed variant replaces the best one so far only when it is faster by more
-// than repeated timings differ (half a percent for the FP32 passes, up to 4 %
-// between two of the FP64 ones, over six constructions of 40 operators):
-// variants that tie would otherwise fall either way from one construction to
-// the next, and with them the summation order, which shows in the results
-// (points to check surfaces in the plain form: its pseudo-inverses turn it into
-// 1e-8; the FP32 near field: 3e-7).  In the FP64 near field it does not (1e-15).
-constexpr float AUTOTUNE_MARGIN_FP32 = 0.99f, AUTOTUNE_MARGIN_FP64 = 0.96f;
+// than repeated timings differ: variants that tie would otherwise fall either
+// way from one construction to the next, and with them the summation order,
+// which shows in the results (points to check surfaces in the plain form: its
+// pseudo-inverses turn it into 1e-8; the FP32 near field: 3e-7; not in the FP64
+// near field, 1e-15).  Timings repeat to half a percent, FP64 ones that depend
+// on where the buffers lie to 3 %.  45 plain operators, four constructions each:
+// with 1 % one choice does not repeat, with none five, with 3 % four.
+constexpr float AUTOTUNE_MARGIN = 0.99f;
 
 // The fastest of `variants` (threads per target; run(v) launches one): each is
 // timed shortly, and, where the choice shows (margin below 1), those within 8 %
 // of the fastest again and longer: there the first in order stays unless
-// another is faster by the margin.  Passes of
-// small operators last 6 to 50 us, of which an event pair resolves half a
-// percent, and a lone launch's own jitter is several: a sample is a row of
-// launches of `span` ms in all, and the fastest sample counts.  (Rows of 0.1 ms
-// spread three times as much as rows of 0.2 to 0.3 ms.)
+// another is faster by the margin.  Passes of small operators last 6 to 50 us,
+// of which an event pair resolves half a percent, and a lone launch's own
+// jitter is several: a sample is a row of launches of `span` ms in all, and the
+// fastest sample counts.  (Rows of 0.1 ms spread three times as much as rows of
+// 0.2 to 0.3 ms.)
 template <typename F>
 int fastest_variant(const std::vector<int>& variants, float margin, cudaStream_t s, F&& run)
 {
@@ -1339,7 +1340,7 @@ void Plan::autotune_p2p()
     const bool mixed = f.mixed && !f.f64;  // FP32 evaluation passes
     if (mixed) TBEM_CK(cudaMemsetAsync(s32.p, 0, sizeof(float) * R * n_src, stream));
     else TBEM_CK(cudaMemsetAsync(s64.p, 0, sizeof(double) * R * n_src, stream));
-    p2p_tpt = fastest_variant({4, 2, 8}, mixed ? AUTOTUNE_MARGIN_FP32 : 1.f, stream, [&](int tpt) {
+    p2p_tpt = fastest_variant({4, 2, 8}, mixed ? AUTOTUNE_MARGIN : 1.f, stream, [&](int tpt) {
         if (mixed)
             eval<float>(p2p, kid, false, false, otree, dobs, 0, *dsrc, 0, s32.p, n_src,
                         nullptr, y64.p, n_obs, nullptr, 1, 1, stream, false, tpt);
@@ -1358,7 +1359,7 @@ void Plan::autotune_p2m()
     const bool mixed = f.mixed && !f.f64;  // FP32 evaluation passes
     if (mixed) TBEM_CK(cudaMemsetAsync(s32.p, 0, sizeof(float) * R * n_src, stream));
     else TBEM_CK(cudaMemsetAsync(s64.p, 0, sizeof(double) * R * n_src, stream));
-    p2m_tpt = fastest_variant({4, 2, 1}, mixed ? AUTOTUNE_MARGIN_FP32 : AUTOTUNE_MARGIN_FP64, stream, [&](int tpt) {
+    p2m_tpt = fastest_variant({4, 2, 1}, AUTOTUNE_MARGIN, stream, [&](int tpt) {
         if (mixed)
             eval<float>(p2m, f.ks_kid, true, false, *stree, *dsrc, f.r_uc, *dsrc, 0, s32.p, n_src,
                         nullptr, nullptr, 0, cu32.p, 0, 1, stream, false, tpt);
