@@ -9,6 +9,8 @@
 // builds the tile tables of this right-hand-side count, so the captured
 // applies make no allocation and no synchronous copy.
 #include <algorithm>
+#include <atomic>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -22,6 +24,7 @@ struct TbemGraph {
     std::vector<cudaEvent_t> joins;
     cudaEvent_t fork = nullptr;
     std::vector<TbemFmm*> ops;                  // not owned
+    std::vector<std::shared_ptr<std::atomic<int>>> counts;  // their live graphs
     int device = 0;
     ~TbemGraph()
     {
@@ -30,6 +33,7 @@ struct TbemGraph {
         const bool own = cudaGetDevice(&prev) == cudaSuccess && prev != device &&
                          cudaSetDevice(device) == cudaSuccess;
         cudaGetLastError();
+        for (auto& c : counts) --*c;
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
         for (auto e : joins) cudaEventDestroy(e);
@@ -105,6 +109,10 @@ void graph_build(TbemGraph& g, TbemFmm* const* ops, int n_ops, const double* con
     TBEM_CK(cudaStreamEndCapture(g.cap, &g.graph));
     TBEM_CK(cudaGraphInstantiate(&g.exec, g.graph, 0));
     g.ops.assign(ops, ops + n_ops);
+    for (TbemFmm* op : g.ops) {
+        ++*op->plan.graphs;
+        g.counts.push_back(op->plan.graphs);
+    }
 }
 
 TbemGraph* graph_new() { return new TbemGraph(); }

@@ -935,6 +935,7 @@ Plan::~Plan()
     for (auto e : event_pool) cudaEventDestroy(e);
     if (h_err) cudaFreeHost(h_err);
     if (cublas) cublasDestroy(cublas);
+    free_retired();
     if (solver) cusolverDnDestroy(solver);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
@@ -3340,6 +3341,12 @@ void Plan::adjoint_compressed(int nrhs, cudaStream_t s)
     eval<T>(p2m_t, F.ks_kid, false, true, S, *dsrc, 0, *dsrc, F.r_uc, nullptr, 0, cu, s64.p, NS, nullptr, 1, nrhs, s, true);
 }
 
+void Plan::free_retired()
+{
+    for (void* p : retired) cudaFree(p);
+    retired.clear();
+}
+
 void Plan::apply(const double* x, double* y, int nrhs, cudaStream_t s, bool adj)
 {
     if (nrhs <= 0) throw Error(TBEM_ERR_ARG, "n_rhs must be > 0");
@@ -3363,6 +3370,11 @@ void Plan::apply(const double* x, double* y, int nrhs, cudaStream_t s, bool adj)
     }
     if (flags_raised())  // raised by an earlier apply
         throw Error(TBEM_ERR_TIMEOUT, "a bounded device wait of an apply gave up");
+    // a captured graph replays the addresses of its capture: while one lives,
+    // buffers that this apply outgrows are kept
+    const bool captured = *graphs > 0;
+    if (!captured && !retired.empty()) free_retired();
+    RetireScope keep(captured ? &retired : nullptr);
     // the right-hand sides run in chunks whose work buffers stay within a
     // fixed budget (the cell buffers grow with cells x right-hand sides)
     const int chunk = rhs_chunk(nrhs);

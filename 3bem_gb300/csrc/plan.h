@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <cusolverDn.h>
 
+#include <atomic>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -69,6 +70,17 @@ struct DeviceGuard {
     DeviceGuard& operator=(const DeviceGuard&) = delete;
 };
 
+// While set (on this thread), released device buffers go there instead of to
+// cudaFree: a captured graph may still address them.
+inline thread_local std::vector<void*>* retire_sink = nullptr;
+struct RetireScope {
+    std::vector<void*>* prev;
+    explicit RetireScope(std::vector<void*>* to) : prev(retire_sink) { retire_sink = to; }
+    ~RetireScope() { retire_sink = prev; }
+    RetireScope(const RetireScope&) = delete;
+    RetireScope& operator=(const RetireScope&) = delete;
+};
+
 // Owning device buffer.
 template <typename T>
 struct DBuf {
@@ -86,7 +98,8 @@ struct DBuf {
     ~DBuf() { release(); }
     void release()
     {
-        if (p) cudaFree(p);
+        if (p && retire_sink) retire_sink->push_back(p);
+        else if (p) cudaFree(p);
         p = nullptr;
         n = 0;
     }
@@ -438,6 +451,12 @@ struct Plan {
     void autotune_p2p();
     void autotune_tc();  // N tile (128 / 64) of the tensor-core translations
     TaskSet p2m_t, p2p_t, m2p_t, p2l_t, l2p_t, m2l_fly_t;
+    // live graphs that captured this operator's applies, and the work buffers
+    // that applies of more right-hand sides have outgrown since (freed by the
+    // next apply without a live graph)
+    std::shared_ptr<std::atomic<int>> graphs = std::make_shared<std::atomic<int>>(0);
+    std::vector<void*> retired;
+    void free_retired();
     // work buffers
     int cap_rhs = 0;
     DBuf<double> io_x, io_y;            // device staging of host data (original order)

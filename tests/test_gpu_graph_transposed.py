@@ -47,3 +47,45 @@ def test_graph_after_transposed_applies(n_rhs):
         ref = op.apply(x)
         assert float((y - ref).norm() / ref.norm()) < 1e-6
         assert all(bool((o == 3.0).all()) for o in others)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp64_compressed"])
+def test_graph_after_applies_of_more_right_hand_sides(precision):
+    """Applies that outgrow the work buffers keep those that a live graph
+    addresses; without a live graph they are freed."""
+    torch = pytest.importorskip("torch")
+    from tbempy import ThreeD, meshes
+    locs, nrm, w = meshes.sphere_points(3)
+    op = ThreeD.FMMOperator(ThreeD.LaplaceSingle(), locs, nrm, locs, nrm, w,
+                            ThreeD.FMMConfig(0.3, 152, 50, 0.05, False), precision=precision)
+    n = len(locs)
+    x = torch.rand(n, dtype=torch.float64, device="cuda")
+    y = torch.zeros(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    g = ThreeD.FMMGraph([op], [x], [y])
+    many = torch.rand((9, n), dtype=torch.float64, device="cuda")
+    tol = {"fp64": 0.0, "mixed": 1e-6, "fp64_compressed": 1e-13}[precision]  # the atomic sums' order
+
+    def replays():
+        x.uniform_(-1, 1)
+        y.zero_()
+        torch.cuda.synchronize()
+        g.launch()
+        torch.cuda.synchronize()
+        ref = op.apply(x)
+        torch.cuda.synchronize()
+        return float((y - ref).norm()) <= tol * float(ref.norm())
+
+    assert replays()
+    for n_rhs in (3, 9):
+        op.apply(many[:n_rhs])
+        op.apply_adjoint(many[:n_rhs])
+        torch.cuda.synchronize()
+        filler = torch.full((1 << 22,), 3.0, device="cuda")  # would take freed memory
+        assert replays() and bool((filler == 3.0).all())
+    del g
+    before = torch.cuda.mem_get_info()[0]
+    ref = op.apply(x)  # frees what the graph had kept
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] >= before
+    assert torch.isfinite(ref).all()
