@@ -2059,7 +2059,7 @@ void Plan::build_mixed_ops(Form& F)
     // compress, else SIMT FP32),
     // 1 SIMT FP32 for all, 2 tensor cores for the M2L only, 3 tensor cores for
     // all, 4 compressed, 5 compressed with the M2L products on tensor cores
-    // (the FP64 compressed form: compressed, FP64 SIMT)
+    // (the FP64 compressed form: compressed, in FP64)
     const int path = F.f64 ? 4 : opt.m2l_path == 0 ? 5 : opt.m2l_path;
     // FP64 copies of the M2L kernel matrices for the compression (compact
     // index), scaled to the root level (see build_m2l_compression)

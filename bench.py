@@ -859,7 +859,7 @@ def nearfield_config(n_subdiv, n_facets, shape, nnz):
                                                       "obs_near_order": 2, "obs_far_order": 2,
                                                       "src_far_order": 2, "n_singular_steps": 8,
                                                       "far_threshold": 3.0},
-            "csr": {"rows": shape[0], "cols": shape[1], "nnz": nnz, "index": "int64", "value": "f64"},
+            "csr": {"rows": shape[0], "cols": shape[1], "nnz": nnz, "index": "int32", "value": "f64"},
             "step": "one CSR apply, 1 RHS",
             "l2": "flushed before every timed step (256 MB write, outside the step timing)"}
 

@@ -63,8 +63,8 @@ extern "C" {
 #define TBEM_PRECISION_FP64 0   /* plain: reference surfaces and formulation, FP64 */
 #define TBEM_PRECISION_MIXED 1  /* precision form: tensor-core M2L/M2M/L2L, FP32 P2P */
 /* The precision form's operators (enclosing surfaces, single-layer
- * equivalent sources, the far field in the M2L SVD bases) applied in FP64 on
- * the SIMT FP64 pipes: the precision form's accuracy against the direct sum
+ * equivalent sources, the far field in the M2L SVD bases) applied in FP64
+ * (m2l_path below): the precision form's accuracy against the direct sum
  * (~1e-7 at the workload orders), but linear to FP64 rounding (its states
  * are well-conditioned check potentials, never the plain form's cancelling
  * equivalent densities) -- the O(N) FP64 residual operator of iterative
@@ -96,9 +96,12 @@ typedef struct {
                               2 tcgen05 3xBF16 for the uncompressed M2L only,
                               3 tcgen05 3xBF16 for M2L, M2M and L2L,
                               4 SVD-compressed far field on the SIMT FP32 pipes,
-                              5 as 4 with all M2L products on tcgen05 3xBF16;
+                              5 as 4 with all M2L products on tcgen05 3xBF16
+                                (transposed applies: FP32 on every path);
                               FP64 compressed form: 4 the M2L on the FP64 pipe,
-                              else through exact digit planes on tcgen05          */
+                              else on tcgen05 through digit planes that hold
+                              products to 2^-58 of a row's and a column's largest
+                              entries, where their memory can be spared           */
     int p2p_block;         /* 0 auto; else threads per target in the P2P kernel (1,2,4,8) */
     int host_only;         /* 1: build trees and task lists only (no device use);
                               apply calls then fail with TBEM_ERR_STATE            */
@@ -269,7 +272,8 @@ int tbem_fmm_setup_times(const TbemFmm* h, const char** names, double* seconds, 
  * candidates 2, 4, 8 at creation unless TbemGpuOptions.p2p_block fixed it). */
 long tbem_fmm_p2p_block(const TbemFmm* h);
 /* N tile (columns) of the precision form's tensor-core translations, chosen
- * by timing the 128- and 64-column shapes at creation (0 when unused). */
+ * by timing the shapes at creation with one right-hand side (0 when unused);
+ * with several, groups that fill 128 columns take 128 where 64 was chosen. */
 long tbem_fmm_tc_tile(const TbemFmm* h);
 
 /* Ranks of the SVD-compressed M2L (input side, output side); both 0 when
@@ -284,8 +288,9 @@ int tbem_fmm_m2l_ranks(const TbemFmm* h, long* r_in, long* r_out);
  * device memory: the graph replays these addresses.  Each operator first
  * runs one ordinary apply (writing y[i]) that sizes its buffers; nothing is
  * allocated while capturing.  An operator's buffers are shared by its
- * applies and its graphs: do not run them concurrently.  Phase timing must be
- * off. */
+ * applies and its graphs: do not run them concurrently.  Between replays any
+ * apply may run: buffers that the graph addresses are kept while it lives.
+ * Phase timing must be off. */
 typedef struct TbemGraph TbemGraph;
 int tbem_fmm_graph_create(TbemFmm* const* ops, int n_ops, const double* const* x,
                           double* const* y, int n_rhs, int adjoint, TbemGraph** out);
